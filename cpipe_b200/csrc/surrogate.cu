@@ -17,10 +17,11 @@
 // Kernels.
 //   sg_prep_kernel   RGBA frame(s) -> a0 (noise map from the per-image model)
 //   sg_conv_kernel   one 8x16-pixel output tile per CTA iteration (4 warps, a
-//                    row pair each), persistent over tiles; the input tile with
-//                    its 1-pixel halo and all weights are staged in shared
-//                    memory (rows padded to 80 B / 592 B so ldmatrix is
-//                    conflict free); A and B fragments by ldmatrix,
+//                    row pair each), persistent over tiles; the input tiles with
+//                    their 1-pixel halo (two buffers: the next tile's cp.async
+//                    copies run behind this tile's products) and all weights
+//                    are staged in shared memory (rows padded to 80 B / 592 B
+//                    so ldmatrix is conflict free); A and B fragments by ldmatrix,
 //                    mma.sync.m16n8k16 bf16 -> f32.  Epilogues: bias + ReLU ->
 //                    bf16; ReLU-mask of the backward pass -> bf16; residual
 //                    add -> RGBA frame; residual + MSE loss gradient (training).
@@ -29,7 +30,13 @@
 //   sg_wgrad_kernel  dW[co][k] = sum_p dY[p][co] * A[p][k]: the same tiles,
 //                    A^T and the im2col operand by transposing ldmatrix,
 //                    per-CTA register accumulation over its tiles, then one
-//                    atomic add per weight; bias gradients alongside.
+//                    two-wide atomic add per weight pair; bias gradients as a
+//                    product with a column of ones.
+// Training step, 16 x 256 x 256 (B200): 2.80 -> 1.70 ms.  It was bound by the
+// latency of the tiles' loads between two barriers (hidden conv 81 -> 69 us,
+// masked 116 -> 72, weight gradient 161 -> 87 with the copies a tile ahead), by
+// one warp adding the bias gradient, and by the loss's single atomic (237 -> 58).
+// What bounds it now is mma.sync and its ldmatrix reads (36 us of a hidden layer).
 //   sg_adam_kernel   Adam on the FP32 master parameters (blob order), after a
 //                    global gradient-norm clip (sg_gradnorm_kernel); a step
 //                    with a non-finite gradient is skipped.
@@ -142,10 +149,45 @@ struct ConvShape {
     static constexpr int NT = COUT / 8;
 };
 
+// Asynchronous copies of a tile into shared memory (16 bytes each, zeros where
+// the source lies outside the frame): the next tile's copies run behind the
+// current tile's products.
+__device__ __forceinline__ void copy16(bf16* dst, const bf16* src, bool inside) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(inside ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copies_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory");
+}
+struct TileGrid {
+    int tiles_x, per_img, tiles;
+    __device__ __forceinline__ TileGrid(int n, int h, int w)
+        : tiles_x((w + kTileW - 1) / kTileW), per_img(tiles_x * ((h + kTileH - 1) / kTileH)), tiles(per_img * n) {}
+    __device__ __forceinline__ void at(int tile, int* img, int* y0, int* x0) const {
+        *img = tile / per_img;
+        const int r = tile - *img * per_img;
+        *y0 = (r / tiles_x) * kTileH;
+        *x0 = (r % tiles_x) * kTileW;
+    }
+};
+// The 10 x 18-pixel halo of the tile at (y0, x0), XS elements per pixel.
+template <int CIN, int XS>
+__device__ __forceinline__ void copy_halo(bf16* s_x, const bf16* x, int img, int y0, int x0, int h, int w) {
+    const bf16* xin = x + (size_t)img * h * w * CIN;
+    for (int i = threadIdx.x; i < kHaloPix * (CIN / 8); i += blockDim.x) {
+        const int pix = i / (CIN / 8), q = i - pix * (CIN / 8);
+        const int gy = y0 + pix / kHaloW - 1, gx = x0 + pix % kHaloW - 1;
+        const bool inside = gy >= 0 && gy < h && gx >= 0 && gx < w;
+        copy16(&s_x[pix * XS + q * 8], inside ? xin + ((size_t)gy * w + gx) * CIN + q * 8 : x, inside);
+    }
+}
+
 template <int CIN, int COUT, int EPI, class T>
 __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
     using S = ConvShape<CIN, COUT>;
-    __shared__ __align__(16) bf16 s_x[kHaloPix * S::XS];
+    __shared__ __align__(16) bf16 s_xb[2][kHaloPix * S::XS];
     __shared__ __align__(16) bf16 s_w[COUT * S::WS];
     __shared__ float s_bias[COUT];
     for (int i = threadIdx.x; i < COUT * (S::KP / 8); i += blockDim.x) {
@@ -154,22 +196,25 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
     }
     if (threadIdx.x < COUT) s_bias[threadIdx.x] = (a.bias && (int)threadIdx.x < a.cout_real) ? a.bias[threadIdx.x] : 0.0F;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_x = (a.w_px + kTileW - 1) / kTileW, tiles_y = (a.h + kTileH - 1) / kTileH;
-    const int per_img = tiles_x * tiles_y, tiles = per_img * a.n;
+    const TileGrid tg(a.n, a.h, a.w_px);
     const long long npx_img = (long long)a.h * a.w_px;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int img = tile / per_img, r = tile - img * per_img;
-        const int y0 = (r / tiles_x) * kTileH, x0 = (r % tiles_x) * kTileW;
-        __syncthreads();
-        const bf16* xin = a.x + (size_t)img * npx_img * CIN;
-        for (int i = threadIdx.x; i < kHaloPix * (CIN / 8); i += blockDim.x) {
-            const int pix = i / (CIN / 8), q = i - pix * (CIN / 8);
-            const int gy = y0 + pix / kHaloW - 1, gx = x0 + pix % kHaloW - 1;
-            uint4 v = make_uint4(0U, 0U, 0U, 0U);
-            if (gy >= 0 && gy < a.h && gx >= 0 && gx < a.w_px)
-                v = *reinterpret_cast<const uint4*>(xin + ((size_t)gy * a.w_px + gx) * CIN + q * 8);
-            *reinterpret_cast<uint4*>(&s_x[pix * S::XS + q * 8]) = v;
+    float sq = 0.0F;  // kEpiLoss: this thread's squared errors over all of the CTA's tiles
+    int img, y0, x0, buf = 0;
+    if ((int)blockIdx.x < tg.tiles) {
+        tg.at(blockIdx.x, &img, &y0, &x0);
+        copy_halo<CIN, S::XS>(s_xb[0], a.x, img, y0, x0, a.h, a.w_px);
+    }
+    copies_commit();
+    for (int tile = blockIdx.x; tile < tg.tiles; tile += gridDim.x, buf ^= 1) {
+        tg.at(tile, &img, &y0, &x0);
+        const bf16* s_x = s_xb[buf];
+        if (tile + (int)gridDim.x < tg.tiles) {
+            int nimg, ny0, nx0;
+            tg.at(tile + gridDim.x, &nimg, &ny0, &nx0);
+            copy_halo<CIN, S::XS>(s_xb[buf ^ 1], a.x, nimg, ny0, nx0, a.h, a.w_px);
         }
+        copies_commit();
+        copies_wait<1>();
         __syncthreads();
         float acc[2][S::NT][4];
 #pragma unroll
@@ -178,7 +223,24 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
             for (int j = 0; j < S::NT; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[mt][j][e] = 0.0F;
-        const int mi = lane >> 3, rr = lane & 7;
+        const int mi = lane >> 3, rr = lane & 7, g = lane >> 2, q = lane & 3;
+        // kEpiMask: the gate's activations are asked for here, so that they
+        // arrive behind the products
+        __nv_bfloat162 gate[EPI == kEpiMask ? 2 : 1][2][S::NT];
+        if constexpr (EPI == kEpiMask) {
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int gy = y0 + warp * 2 + mt, gx = x0 + g + 8 * half;
+                    const bool inside = gy < a.h && gx < a.w_px;
+                    const bf16* src = a.mask + ((long long)img * npx_img + (long long)gy * a.w_px + gx) * COUT + 2 * q;
+#pragma unroll
+                    for (int j = 0; j < S::NT; ++j)
+                        gate[mt][half][j] = inside ? *reinterpret_cast<const __nv_bfloat162*>(src + 8 * j)
+                                                   : __nv_bfloat162{};
+                }
+        }
 #pragma unroll
         for (int ks = 0; ks < S::KSTEPS; ++ks) {
             uint32_t af[2][4];
@@ -214,8 +276,8 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
                 }
             }
         }
+        __syncthreads();  // every warp is done with this tile's buffer (the next round copies into it)
         // epilogue: acc[mt][j][0..1] at pixel (row, g), channels 8j+2q+{0,1}; [2..3] at pixel g+8
-        const int g = lane >> 2, q = lane & 3;
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             const int gy = y0 + warp * 2 + mt;
@@ -234,7 +296,7 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
                                 v0 = fmaxf(v0 + s_bias[c], 0.0F);
                                 v1 = fmaxf(v1 + s_bias[c + 1], 0.0F);
                             } else {
-                                const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162*>(a.mask + p * COUT + c);
+                                const __nv_bfloat162 mk = gate[mt][half][j];
                                 v0 = __low2float(mk) > 0.0F ? v0 : 0.0F;
                                 v1 = __high2float(mk) > 0.0F ? v1 : 0.0F;
                             }
@@ -254,12 +316,11 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
                                                  src);
                         }
                     } else {
-                        float sq = 0.0F;
                         if (inside && q == 0) {
                             const Rgba x = load_rgba(static_cast<const __half*>(a.rgba) + 4 * p);
                             const Rgba t = load_rgba(a.target + 4 * p);
                             const float d0 = (x.r + c0) - t.r, d1 = (x.g + c1) - t.g, d2 = (x.b + c2) - t.b;
-                            sq = d0 * d0 + d1 * d1 + d2 * d2;
+                            sq += d0 * d0 + d1 * d1 + d2 * d2;
                             __nv_bfloat162 v[4];
                             v[0] = __floats2bfloat162_rn(d0 * a.grad_scale, d1 * a.grad_scale);
                             v[1] = __floats2bfloat162_rn(d2 * a.grad_scale, 0.0F);
@@ -267,13 +328,17 @@ __global__ void __launch_bounds__(128) sg_conv_kernel(ConvArgs a) {
                             v[3] = v[2];
                             *reinterpret_cast<uint4*>(a.y + p * 8) = *reinterpret_cast<const uint4*>(v);
                         }
-#pragma unroll
-                        for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFU, sq, off);
-                        if (lane == 0 && sq != 0.0F) atomicAdd(a.loss, sq);
                     }
                 }
             }
         }
+    }
+    if constexpr (EPI == kEpiLoss) {
+        // one add per warp and launch: an add per 16 pixels kept every warp of
+        // the device on one address (237 us of the layer's 16 x 256 x 256 pass)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFU, sq, off);
+        if (lane == 0 && sq != 0.0F) atomicAdd(a.loss, sq);
     }
 }
 
@@ -287,18 +352,30 @@ struct WgradArgs {
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) sg_wgrad_kernel(WgradArgs a) {
+__global__ void __launch_bounds__(128, 4) sg_wgrad_kernel(WgradArgs a) {
     using S = ConvShape<CIN, COUT>;
     constexpr int DS = COUT == 32 ? 40 : 16;  // dY smem pixel stride; COUT 8 is zero padded to 16 rows of A
     constexpr int MT = COUT == 32 ? 2 : 1;
     constexpr int NTOT = 9 * CIN / 8;         // n8 tiles over the real K
     constexpr int NPW = (NTOT + 3) / 4;       // per warp
-    __shared__ __align__(16) bf16 s_x[kHaloPix * S::XS];
-    __shared__ __align__(16) bf16 s_d[kTileH * kTileW * DS];
+    constexpr int XN = kHaloPix * S::XS, DN = kTileH * kTileW * DS;
+    extern __shared__ __align__(16) bf16 s_tiles[];  // two buffers of input halo and gradient tile
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_x = (a.w_px + kTileW - 1) / kTileW, tiles_y = (a.h + kTileH - 1) / kTileH;
-    const int per_img = tiles_x * tiles_y, tiles = per_img * a.n;
-    const long long npx_img = (long long)a.h * a.w_px;
+    const TileGrid tg(a.n, a.h, a.w_px);
+    auto stage = [&](int tile, int buf) {
+        int img, y0, x0;
+        tg.at(tile, &img, &y0, &x0);
+        bf16* s_x = s_tiles + buf * (XN + DN);
+        bf16* s_d = s_x + XN;
+        copy_halo<CIN, S::XS>(s_x, a.x, img, y0, x0, a.h, a.w_px);
+        const bf16* din = a.dy + (size_t)img * a.h * a.w_px * COUT;
+        for (int i = threadIdx.x; i < kTileH * kTileW * (DS / 8); i += blockDim.x) {
+            const int pix = i / (DS / 8), qq = i - pix * (DS / 8);
+            const int gy = y0 + pix / kTileW, gx = x0 + pix % kTileW;
+            const bool inside = qq < COUT / 8 && gy < a.h && gx < a.w_px;
+            copy16(&s_d[pix * DS + qq * 8], inside ? din + ((size_t)gy * a.w_px + gx) * COUT + qq * 8 : a.dy, inside);
+        }
+    };
     float acc[MT][NPW][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -306,39 +383,35 @@ __global__ void __launch_bounds__(128) sg_wgrad_kernel(WgradArgs a) {
         for (int j = 0; j < NPW; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[mt][j][e] = 0.0F;
-    float bsum = 0.0F;
+    // bias gradients: the product of dY^T with a column of ones, tile rows dealt
+    // out to the warps (one warp adding 128 pixels one by one held the others up)
+    float bacc[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bacc[mt][e] = 0.0F;
+    constexpr uint32_t kOnes = 0x3F803F80U;  // bf16 (1, 1)
     const int mi = lane >> 3, rr = lane & 7;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int img = tile / per_img, r = tile - img * per_img;
-        const int y0 = (r / tiles_x) * kTileH, x0 = (r % tiles_x) * kTileW;
+    int buf = 0;
+    if ((int)blockIdx.x < tg.tiles) stage(blockIdx.x, 0);
+    copies_commit();
+    for (int tile = blockIdx.x; tile < tg.tiles; tile += gridDim.x, buf ^= 1) {
+        const bf16* s_x = s_tiles + buf * (XN + DN);
+        const bf16* s_d = s_x + XN;
+        if (tile + (int)gridDim.x < tg.tiles) stage(tile + gridDim.x, buf ^ 1);
+        copies_commit();
+        copies_wait<1>();
         __syncthreads();
-        const bf16* xin = a.x + (size_t)img * npx_img * CIN;
-        for (int i = threadIdx.x; i < kHaloPix * (CIN / 8); i += blockDim.x) {
-            const int pix = i / (CIN / 8), qq = i - pix * (CIN / 8);
-            const int gy = y0 + pix / kHaloW - 1, gx = x0 + pix % kHaloW - 1;
-            uint4 v = make_uint4(0U, 0U, 0U, 0U);
-            if (gy >= 0 && gy < a.h && gx >= 0 && gx < a.w_px)
-                v = *reinterpret_cast<const uint4*>(xin + ((size_t)gy * a.w_px + gx) * CIN + qq * 8);
-            *reinterpret_cast<uint4*>(&s_x[pix * S::XS + qq * 8]) = v;
-        }
-        const bf16* din = a.dy + (size_t)img * npx_img * COUT;
-        for (int i = threadIdx.x; i < kTileH * kTileW * (DS / 8); i += blockDim.x) {
-            const int pix = i / (DS / 8), qq = i - pix * (DS / 8);
-            const int gy = y0 + pix / kTileW, gx = x0 + pix % kTileW;
-            uint4 v = make_uint4(0U, 0U, 0U, 0U);
-            if (qq < COUT / 8 && gy < a.h && gx < a.w_px)
-                v = *reinterpret_cast<const uint4*>(din + ((size_t)gy * a.w_px + gx) * COUT + qq * 8);
-            *reinterpret_cast<uint4*>(&s_d[pix * DS + qq * 8]) = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < COUT)
-            for (int p = 0; p < kTileH * kTileW; ++p) bsum += __bfloat162float(s_d[p * DS + threadIdx.x]);
 #pragma unroll
         for (int ks = 0; ks < kTileH; ++ks) {  // k-step = one tile row of 16 pixels
             uint32_t af[MT][4];
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
                 ldsm_x4_t(af[mt], &s_d[(ks * kTileW + rr + 8 * (mi >> 1)) * DS + 16 * mt + 8 * (mi & 1)]);
+            if ((ks & 3) == warp) {
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) mma_bf16(bacc[mt], af[mt], kOnes, kOnes);
+            }
 #pragma unroll
             for (int j = 0; j < NPW; ++j) {
                 const int nt = warp * NPW + j;
@@ -352,6 +425,7 @@ __global__ void __launch_bounds__(128) sg_wgrad_kernel(WgradArgs a) {
                 }
             }
         }
+        __syncthreads();
     }
     const int g = lane >> 2, q = lane & 3;
 #pragma unroll
@@ -364,13 +438,20 @@ __global__ void __launch_bounds__(128) sg_wgrad_kernel(WgradArgs a) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int co = 16 * mt + g + 8 * half;
-                if (co < COUT) {
-                    atomicAdd(&a.dw[co * S::KP + k], acc[mt][j][2 * half]);
-                    atomicAdd(&a.dw[co * S::KP + k + 1], acc[mt][j][2 * half + 1]);
-                }
+                if (co < COUT)
+                    atomicAdd(reinterpret_cast<float2*>(&a.dw[co * S::KP + k]),
+                              make_float2(acc[mt][j][2 * half], acc[mt][j][2 * half + 1]));
             }
         }
-    if (threadIdx.x < COUT) atomicAdd(&a.db[threadIdx.x], bsum);
+    if (q == 0) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int co = 16 * mt + g + 8 * half;
+                if (co < COUT) atomicAdd(&a.db[co], bacc[mt][2 * half]);
+            }
+    }
 }
 
 // ------------------------------------------------------------ adam / pack
@@ -546,8 +627,13 @@ static void conv(const ConvArgs& a, long long tiles, cudaStream_t st) {
     sg_conv_kernel<CIN, COUT, EPI, T><<<grid_for(tiles, 4), 128, 0, st>>>(a);
 }
 template <int CIN, int COUT>
-static void wgrad(const WgradArgs& a, long long tiles, cudaStream_t st) {
-    sg_wgrad_kernel<CIN, COUT><<<grid_for(tiles, 4), 128, 0, st>>>(a);
+static cudaError_t wgrad(const WgradArgs& a, long long tiles, cudaStream_t st) {
+    constexpr int bytes =
+        2 * (int)sizeof(bf16) * (kHaloPix * ConvShape<CIN, COUT>::XS + kTileH * kTileW * (COUT == 32 ? 40 : 16));
+    // set on every call: the attribute belongs to the current device
+    const cudaError_t e = cudaFuncSetAttribute(sg_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) sg_wgrad_kernel<CIN, COUT><<<grid_for(tiles, 4), 128, bytes, st>>>(a);
+    return e;
 }
 
 static ConvArgs conv_args(const SurrogateNet* s, int l, const bf16* x, bf16* y, int n, int h, int w) {
@@ -833,9 +919,10 @@ int cpipe_surrogate_train_step(cpipe_surrogate* s, const void* d_noisy, const vo
     const bf16* g = net->d_gout;
     for (int l = kLayers - 1; l >= 0; --l) {
         WgradArgs wa{act(l), g, n, height, width, net->d_grad + net->t.goff[l], net->d_grad + net->t.gboff[l]};
-        if (l == kLayers - 1) wgrad<kCh, 8>(wa, tiles, st);
-        else if (l == 0) wgrad<8, kCh>(wa, tiles, st);
-        else wgrad<kCh, kCh>(wa, tiles, st);
+        if (l == kLayers - 1) e = wgrad<kCh, 8>(wa, tiles, st);
+        else if (l == 0) e = wgrad<8, kCh>(wa, tiles, st);
+        else e = wgrad<kCh, kCh>(wa, tiles, st);
+        if (e != cudaSuccess) return cuda_status(e, "surrogate weight gradient");
         if (l == 0) break;
         bf16* gn = net->d_g[l & 1];
         ConvArgs a{};

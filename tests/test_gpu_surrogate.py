@@ -70,6 +70,24 @@ def test_gradients_match_oracle(cuda_device):
     sg.close()
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 8, 16), (2, 9, 17), (1, 129, 600)])
+def test_gradients_match_oracle_over_tile_counts(cuda_device, n, h, w):
+    """One tile, exact tiles, ragged edges, and more tiles than CTAs (646 against 592, so the double-buffered tile
+    loop runs): loss and gradients against the oracle with the bounds of the test above."""
+    rgba, tgt, ab, params = small_problem(3, n=n, h=h, w=w)
+    sg = S.Surrogate(S.to_blob(params))
+    dn, dt = upload_f16(rgba), upload_f16(tgt)
+    loss = sg.train_step(dn.ptr, dt.ptr, ab, n, w, h, 0.0, update=False)
+    grads = sg.gradients()
+    want_loss, want = O.loss_and_grads(params, rgba.astype(np.float32), tgt.astype(np.float32), ab, bf=True)
+    assert abs(loss - want_loss) <= 1e-3 * want_loss, (loss, want_loss)
+    for l, ((gw, gb), (ow, ob)) in enumerate(zip(grads, want)):
+        ew = np.linalg.norm(gw - ow) / max(np.linalg.norm(ow), 1e-30)
+        eb = np.linalg.norm(gb - ob) / max(np.linalg.norm(ob), 1e-30)
+        assert ew < 2e-2 and eb < 2e-2, (l, ew, eb)
+    sg.close()
+
+
 def test_forward_matches_oracle(cuda_device):
     rgba, _, ab, params = small_problem(1, n=2, h=19, w=35)
     n, h, w = rgba.shape[:3]
