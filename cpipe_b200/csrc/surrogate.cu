@@ -8,8 +8,8 @@
 //
 // Layout.  Activations are NHWC bf16: the input a0 has 8 channels (R, G, B,
 // sigma/0.03, four zeros), hidden activations a1..a7 32 channels (post-ReLU).
-// The tcgen05 inference path keeps its hidden activations in 8-channel planes,
-// [n][4][h][w][8] (surrogate_tc.cu); a0 is the same in both layouts.
+// The tcgen05 inference path (surrogate_tc.cu) keeps one hidden activation in
+// device memory, in 8-channel planes, [n][4][h][w][8].
 // Layer l is an implicit GEMM  out[p][co] = sum_k A[p][k] * W[co][k]  with
 // k = tap * CIN + ci (tap = 3*(dy+1) + (dx+1)), K padded to a multiple of 16;
 // the weights are stored [COUT][K] (the col-major B operand of mma).
@@ -690,37 +690,31 @@ static cudaError_t infer(SurrogateNet* s, const void* in, void* out, int n, int 
     cudaError_t e = ensure_acts(s, px, false);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[0], st);
-    if (f16) sg_prep_kernel<__half><<<(unsigned)((px + 255) / 256), 256, 0, st>>>(static_cast<const __half*>(in), s->d_act, d_ab, (long long)h * w, n);
-    else sg_prep_kernel<float><<<(unsigned)((px + 255) / 256), 256, 0, st>>>(static_cast<const float*>(in), s->d_act, d_ab, (long long)h * w, n);
-    if (ev) cudaEventRecord(ev[1], st);
-    if (s->use_tc) {
-        const bf16* cur = s->d_act;
-        bf16* hid = s->d_act + (size_t)px * 8;
-        for (int l = 0; l < kLayers; ++l) {
-            TcConvArgs t{};
-            t.n = n;
-            t.h = h;
-            t.w = w;
-            t.w_rows = cout_pad(l);
-            t.bias = s->d_params + s->t.boff[l];
-            t.cout_real = cout_real(l);
-            t.err = s->d_err;
-            cudaError_t e2;
-            if (l < kLayers - 1) {
-                bf16* nxt = hid + (size_t)(l & 1) * px * kCh;
-                t.y = nxt;
-                e2 = tc_conv(cin_pad(l), kCh, 0, f16, cur, s->d_packed + s->t.fwoff[l], t, st);
-                cur = nxt;
-            } else {
-                t.rgba = in;
-                t.out = out;
-                e2 = tc_conv(kCh, 16, 1, f16, cur, s->d_packed + s->t.fwoff[l], t, st);
+    if (s->use_tc) {  // two kernels of four layers; the events between layers mark the kernel's end
+        TcNetArgs t{};
+        t.n = n;
+        t.h = h;
+        t.w = w;
+        t.rgba = in;
+        t.out = out;
+        t.ab = d_ab;
+        t.sigma_scale = kSigmaScale;
+        t.act = s->d_act;
+        t.err = s->d_err;
+        if (ev) cudaEventRecord(ev[1], st);
+        for (int half = 0; half < 2; ++half) {
+            for (int p = 0; p < 4; ++p) {
+                t.weights[p] = s->d_packed + s->t.fwoff[4 * half + p];
+                t.bias[p] = s->d_params + s->t.boff[4 * half + p];
             }
-            if (e2 != cudaSuccess) return e2;
-            if (ev) cudaEventRecord(ev[l + 2], st);
+            if ((e = tc_net(half == 0, f16, t, st)) != cudaSuccess) return e;
+            for (int p = 0; p < 4 && ev; ++p) cudaEventRecord(ev[4 * half + p + 2], st);
         }
         return cudaGetLastError();
     }
+    if (f16) sg_prep_kernel<__half><<<(unsigned)((px + 255) / 256), 256, 0, st>>>(static_cast<const __half*>(in), s->d_act, d_ab, (long long)h * w, n);
+    else sg_prep_kernel<float><<<(unsigned)((px + 255) / 256), 256, 0, st>>>(static_cast<const float*>(in), s->d_act, d_ab, (long long)h * w, n);
+    if (ev) cudaEventRecord(ev[1], st);
     const bf16* a7 = forward_hidden(s, n, h, w, false, st, ev);
     ConvArgs a = conv_args(s, kLayers - 1, a7, nullptr, n, h, w);
     a.rgba = in;
@@ -763,7 +757,6 @@ SurrogateNet* surrogate_new(const void* blob, size_t size, int* status) {
     if (cudaMemcpy(s->d_params, params, sizeof(float) * s->nparams, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(CPIPE_INTERNAL_ERROR, s);
     if (pack(s, nullptr) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return fail(CPIPE_INTERNAL_ERROR, s);
-    s->use_tc = tc_conv_available();
     if (status) *status = CPIPE_OK;
     return s;
 }
@@ -840,10 +833,6 @@ int cpipe_surrogate_denoise(cpipe_surrogate* s, const void* d_in, void* d_out, i
 
 int cpipe_surrogate_set_engine(cpipe_surrogate* s, int engine) {
     if (!s || (engine != 0 && engine != 1)) return CPIPE_BAD_INDEX;
-    if (engine == 1 && !tc_conv_available()) {
-        set_error("surrogate: %s", "tensor-map encoder unavailable for the tcgen05 engine");
-        return CPIPE_UNSUPPORTED;
-    }
     s->net->use_tc = engine == 1;
     return CPIPE_OK;
 }
@@ -855,8 +844,8 @@ int cpipe_surrogate_check(cpipe_surrogate* s) {
     if (st != CPIPE_OK) return st;
     if (cudaMemcpy(&err, s->net->d_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return CPIPE_INTERNAL_ERROR;
     if (err) {
-        set_error("surrogate: tcgen05 pipeline wait ran out (%s)", err == 1 ? "input stage" : err == 2 ? "tile load"
-                                                                    : err == 3 ? "accumulator" : "MMA completion");
+        set_error("surrogate: tcgen05 pipeline wait ran out (%s)", err == 1 ? "input row" : err == 2 ? "accumulator"
+                                                                    : err == 3 ? "input ring" : "epilogue");
         return CPIPE_INTERNAL_ERROR;
     }
     return CPIPE_OK;
@@ -874,8 +863,18 @@ int cpipe_surrogate_profile(cpipe_surrogate* s, const void* d_in, void* d_out, i
     if (status == CPIPE_OK && e == cudaSuccess)
         e = infer(s->net, d_in, d_out, n, height, width, f16 != 0, s->net->d_ab, st, ev);
     if (status == CPIPE_OK && e == cudaSuccess) e = cudaEventSynchronize(ev[kLayers + 1]);
-    if (status == CPIPE_OK && e == cudaSuccess)
+    if (status == CPIPE_OK && e == cudaSuccess) {
         for (int k = 0; k <= kLayers; ++k) cudaEventElapsedTime(&ms[k], ev[k], ev[k + 1]);
+        if (s->net->use_tc)  // a kernel's four layers share its time by their multiply-adds
+            for (int half = 0; half < 2; ++half) {
+                float* t = ms + 1 + 4 * half;
+                const float sum = t[0] + t[1] + t[2] + t[3];
+                float macs = 0.0F;
+                for (int p = 0; p < 4; ++p) macs += (float)(cin_real(4 * half + p) * cout_real(4 * half + p));
+                for (int p = 0; p < 4; ++p)
+                    t[p] = sum * (float)(cin_real(4 * half + p) * cout_real(4 * half + p)) / macs;
+            }
+    }
     for (auto& x : ev)
         if (x) cudaEventDestroy(x);
     return status != CPIPE_OK ? status : cuda_status(e, "surrogate profile");

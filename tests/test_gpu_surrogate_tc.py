@@ -55,6 +55,23 @@ def test_tcgen05_matches_mma_and_oracle(cuda_device, n, h, w):
     sg.close()
 
 
+# strips of up to 122 columns and CTAs of at least 8 rows: one strip exactly, one column more, three strips, rows
+# dealt out across frames and strips, fewer rows than a layer's reach, one row
+@pytest.mark.parametrize("n,h,w", [(1, 9, 122), (2, 17, 123), (1, 40, 245), (3, 7, 260), (1, 2, 130), (1, 1, 300),
+                                   (1, 301, 5)])
+def test_tcgen05_strips_match_mma(cuda_device, n, h, w):
+    rng = np.random.default_rng(h * 1000 + w)
+    x = rng.uniform(0.02, 0.95, (n, h, w, 4)).astype(np.float16)
+    ab = np.array([(4e-3, 4e-5), (1e-3, 1e-5), (8e-3, 9e-5)][:n], np.float32)
+    params = [(W, (b + rng.normal(0, 0.02, b.shape)).astype(np.float32)) for W, b in S.init_params(n + h)]
+    params[-1] = (params[-1][0] * 10.0, params[-1][1])
+    sg = S.Surrogate(S.to_blob(params))
+    tc, mma = run(sg, "tcgen05", x, ab), run(sg, "mma", x, ab)
+    np.testing.assert_array_equal(tc[..., 3], x[..., 3].astype(np.float32))
+    close(tc[..., :3], mma[..., :3], f"tcgen05 vs mma {n}x{h}x{w}")
+    sg.close()
+
+
 def test_tcgen05_float32_frames(cuda_device):
     rng = np.random.default_rng(7)
     x = rng.uniform(0.02, 0.95, (1, 24, 40, 4)).astype(np.float32)
