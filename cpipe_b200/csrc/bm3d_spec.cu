@@ -24,12 +24,8 @@
 // Kernels (all FP32 on the CUDA cores; the transforms use explicit fused
 // multiply-adds, the library being built without contraction):
 //   bm3d_prep_kernel    RGBA -> Y,U,V planes + 8-bit matching luminance
-//   bm3d_match_kernel   one thread per reference block; the search region of a
-//                       16x16 tile of references is staged in shared memory as
-//                       four byte-shifted word copies so every 4-pixel chunk is
-//                       one aligned 32-bit load; distances with byte-SIMD
-//                       |a-b| and dp4a (exact integers); a sorted register list
-//                       keeps the 15 best (d << 11 | window index) keys
+//   bm3d_match_kernel   block distances on the integer tensor cores, two passes
+//                       (a bound, then the candidates it lets through)
 //   bm3d_filter_kernel  one warp per group and channel: lane = (block, row
 //                       half); row DCT in registers, column DCT through a warp
 //                       shared buffer, Haar along the group with warp shuffles;
@@ -45,6 +41,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/cpipe_node_abi.h"
 #include "kernels.h"
@@ -109,7 +106,8 @@ __global__ void bm3d_prep_kernel(Img in, float* __restrict__ yuv, uint8_t* __res
 
 // ------------------------------------------------------------------ match
 struct MatchArgs {
-    int w, h, nrx, nry, nstep, R, ns, n2, wpr, rows;  // h: one image's height (blockIdx.z = image)
+    int w, h, nrx, nry, nstep, R, ns, n2;  // h: one image's height (blockIdx.z = image)
+    int tile, wpr, plane, epitch;          // references per CTA edge; pitches of the staged region (words)
     uint32_t dthr;
     const uint8_t* q;
     uint32_t* list;
@@ -117,117 +115,348 @@ struct MatchArgs {
     const int* gate;
 };
 
-constexpr int kMatchTile = 16;  // reference blocks per CTA edge (one thread each)
-constexpr int kMatchWprStd = 24;  // words per staged row for the 39x39 window at step 3
+constexpr int kMatchQueue = 32;  // candidates a reference may have waiting
+constexpr int kMatchStride = kMatchQueue + 1;  // words per reference: the queue and its length
 
-// WPR > 0: words per staged row fixed at compile time (the standard 39x39
-// window), 0: taken from the arguments.
-template <int WPR>
-__global__ void __launch_bounds__(256) bm3d_match_kernel(MatchArgs a) {
+// The distances come from the integer tensor cores.  With the block energies
+// E(p) = sum of q^2 over the 8x8 block at p, a reference r and a candidate c
+// are d = E(r) + E(c) - 2 r.c apart, and r.c for 16 references and 8
+// neighbouring candidates is one m16n8k32 product for each half of a block.
+// The candidates' half energies go in as the product's addend: what comes out
+// is s = r.c - ceil(E(c) / 2), and d = E(r) - 2 s - (E(c) & 1).
+__device__ __forceinline__ void mma_u8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
+}
+
+// A warp's references are 8 columns (lane / 4) x 4 rows (j).  It walks the union
+// of their windows in tiles of 8 columns and one row, twice:
+//   pass 1 keeps the largest s of 32 buckets a reference.  The 16th largest
+//          bucket bounds the 15 best candidates (one bucket may hold nothing
+//          better than the reference itself), and lets about 20 of 1521
+//          candidates through;
+//   pass 2 computes the same distances again, in raster order, and queues what
+//          the bound lets through with its (distance, window index) key; a lane
+//          sorts one reference's queue.  A queue about to overflow (flat areas
+//          tie everywhere) is sorted in early; from then on only a smaller
+//          distance than the 15th best passes.
+//
+// Shared memory: the search region of the CTA's references as four byte-shifted
+// word copies (any 4 pixels are one aligned word; pitches 4 mod 8 and 8 mod 32
+// keep the fragments' loads free of bank conflicts), the energies, the queues.
+//
+// Bound by instruction issue (half the cycles, 16 warps an SM): the products
+// take a fifth of the integer tensor pipe, the rest is two to three
+// instructions per distance, half of them for pairs outside a window, and the
+// queueing of what passes.  12 MP chain frame, per stage: 4.7 -> 3.7 ms; 16
+// tiles of 256 x 256: 636 -> 436 us, against a thread per reference with
+// byte-SIMD |a - b|, dp4a and a sorted list.  (Visiting columns first, and
+// with them letting equal distances through, cost 9 ms on the same frame.)
+__global__ void __launch_bounds__(256, 2) bm3d_match_kernel(MatchArgs a) {
     extern __shared__ uint32_t s_w[];
-    const int wpr = WPR > 0 ? WPR : a.wpr;
     if (gated_off(a.gate)) return;
     const int img = blockIdx.z, row0 = img * a.h;  // images are stacked in rows
-    const int i0 = blockIdx.x * kMatchTile, j0 = blockIdx.y * kMatchTile;
-    const int iL = min(i0 + kMatchTile - 1, a.nrx - 1), jL = min(j0 + kMatchTile - 1, a.nry - 1);
+    const int i0 = blockIdx.x * a.tile, j0 = blockIdx.y * a.tile;
+    const int iL = min(i0 + a.tile - 1, a.nrx - 1), jL = min(j0 + a.tile - 1, a.nry - 1);
     const int rx0 = max(0, refpos(i0, a.w, a.nstep) - a.R);
     const int rx1 = min(a.w, refpos(iL, a.w, a.nstep) + a.R + 8);
     const int ry0 = row0 + max(0, refpos(j0, a.h, a.nstep) - a.R);
     const int ry1 = row0 + min(a.h, refpos(jL, a.h, a.nstep) + a.R + 8);
     const int RW = rx1 - rx0, RH = ry1 - ry0;
-    const int plane = a.rows * wpr;  // words per shifted copy
-    // Copy s, row r, word k holds region bytes 4k+s .. 4k+s+3 (little endian).
-    for (int idx = threadIdx.x; idx < 4 * RH * wpr; idx += blockDim.x) {
-        const int s = idx / (RH * wpr), rem = idx - s * RH * wpr;
-        const int r = rem / wpr, k = rem - r * wpr;
-        const uint8_t* row = a.q + (size_t)(ry0 + r) * a.w + rx0;
-        const int c0 = 4 * k + s;
-        uint32_t word = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int cc = c0 + b;
-            word |= (cc < RW ? (uint32_t)row[cc] : 0U) << (8 * b);
-        }
-        s_w[s * plane + r * wpr + k] = word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    int* s_e = reinterpret_cast<int*>(s_w + 4 * a.plane);  // minus the block energies
+    uint32_t* s_q = reinterpret_cast<uint32_t*>(s_e + (size_t)a.epitch * (RH - 7)) + warp * 32 * kMatchStride;
+
+    // copy 0: the region's bytes; copy s, row r, word k holds region bytes 4k+s .. 4k+s+3
+    uint8_t* bytes = reinterpret_cast<uint8_t*>(s_w);
+    for (int r = warp; r < RH; r += warps) {
+        const uint8_t* src = a.q + (size_t)(ry0 + r) * a.w + rx0;
+        for (int c = lane; c < 4 * a.wpr; c += 32) bytes[4 * r * a.wpr + c] = c < RW ? src[c] : (uint8_t)0;
     }
     __syncthreads();
-    const int i = i0 + (int)(threadIdx.x % kMatchTile), j = j0 + (int)(threadIdx.x / kMatchTile);
-    if (i >= a.nrx || j >= a.nry) return;
-    const int x = refpos(i, a.w, a.nstep), y = row0 + refpos(j, a.h, a.nstep);
-    uint32_t rw[16];
-    {
-        const int c = x - rx0;
-        const uint32_t* p = s_w + (c & 3) * plane + (y - ry0) * wpr + (c >> 2);
+    for (int r = warp; r < RH; r += warps)
+        for (int k = lane; k < a.wpr; k += 32) {
+            const uint32_t* p = s_w + r * a.wpr + k;
+            const uint32_t lo = p[0], hi = k + 1 < a.wpr ? p[1] : 0U;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            rw[2 * r] = p[r * wpr];
-            rw[2 * r + 1] = p[r * wpr + 1];
+            for (int s = 1; s < 4; ++s) s_w[s * a.plane + r * a.wpr + k] = __funnelshift_r(lo, hi, 8 * s);
+        }
+    __syncthreads();
+    // energies: a thread walks down a column with the last eight rows' sums in a ring
+    {
+        constexpr int kRows = 16;
+        const int cols = RW - 7, rows = RH - 7;  // block positions
+        // (columns past the last position read as zero: s and v stay below 2^22 there)
+        for (int i = threadIdx.x; i < rows * (a.epitch - cols); i += blockDim.x) {
+            const int y = i / (a.epitch - cols);
+            s_e[y * a.epitch + cols + i - y * (a.epitch - cols)] = 0;
+        }
+        for (int item = threadIdx.x; item < cols * ((rows + kRows - 1) / kRows); item += blockDim.x) {
+            const int seg = item / cols, x = item - seg * cols;
+            const int y0 = seg * kRows, y1 = min(rows, y0 + kRows);
+            const uint32_t* p = s_w + (x & 3) * a.plane + (x >> 2);
+            auto row_energy = [&](int y) {
+                const uint32_t w0 = p[y * a.wpr], w1 = p[y * a.wpr + 1];
+                return (int)__dp4a(w1, w1, __dp4a(w0, w0, 0U));
+            };
+            int e = 0;
+            for (int y = y0; y < y0 + 8; ++y) e += row_energy(y);
+            for (int y = y0; y < y1; ++y) {
+                s_e[y * a.epitch + x] = -e;
+                if (y + 1 < y1) e += row_energy(y + 8) - row_energy(y);
+            }
         }
     }
+    __syncthreads();
+
+    const int g = lane >> 2, q = lane & 3;
+    const int wi = i0 + (warp % (a.tile / 8)) * 8, wj = j0 + (warp / (a.tile / 8)) * 4;  // a warp takes 8 x 4 references
+    if (wi >= a.nrx || wj >= a.nry) return;  // (whole warps; no barrier follows)
+    // positions of the lane's references (column g, rows j); past the last one the last again
+    const int x = refpos(min(wi + g, a.nrx - 1), a.w, a.nstep);
+    int y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) y[j] = row0 + refpos(min(wj + j, a.nry - 1), a.h, a.nstep);
+    const int ylo = max(row0, y[0] - a.R), yhi = min(row0 + a.h - 8, y[3] + a.R);
+    const int xlo = max(0, refpos(wi, a.w, a.nstep) - a.R);
+    const int xhi = min(a.w - 8, refpos(min(wi + 7, a.nrx - 1), a.w, a.nstep) + a.R);
+    const int xs = rx0 + ((xlo - rx0) & ~1);  // even in the region, so two energies are one load
+
+    // A fragments: K = 4 bytes (row q / 2, half q % 2) of two block rows; rows 2, 4, 6 further on
+    uint32_t af[4][4];
+    int er[4];
+    {
+        const int c = x - rx0 + 4 * (q & 1);
+        const uint32_t* p = s_w + (c & 3) * a.plane + (c >> 2) + (q >> 1) * a.wpr;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = y[j] - ry0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) af[j][k] = p[(r + 2 * k) * a.wpr];
+            er[j] = -s_e[r * a.epitch + x - rx0];
+        }
+    }
+    constexpr int kNone = -0x20000000;  // below every s
+    // a candidate may still enter the list when v = E(r) - d = 2 r.c - E(c) is
+    // above lim[j]; first from the match threshold
+    int lim[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) lim[j] = er[j] - (int)a.dthr - 1;
     uint32_t keys[15];
 #pragma unroll
     for (int m = 0; m < 15; ++m) keys[m] = 0xFFFFFFFFU;
-    const int ylo = max(row0, y - a.R), yhi = min(row0 + a.h - 8, y + a.R);
-    const int xlo = max(0, x - a.R), xhi = min(a.w - 8, x + a.R);
-    if (a.n2 > 1) {
-        // Columns of the search window outer, rows inner: the candidate's eight
-        // rows sit in a register ring (slot = row & 7, rows counted from ylo), so
-        // each candidate loads one new row.  Keys are unique (distance, window
-        // index), so the sorted list does not depend on the visiting order.
-        const int ny = yhi - ylo + 1;
-        for (int xx = xlo; xx <= xhi; ++xx) {
-            const int c = xx - rx0;
-            const uint32_t* colp = s_w + (c & 3) * plane + (ylo - ry0) * wpr + (c >> 2);
-            const uint32_t wcol = (uint32_t)((ylo - y + a.R) * a.ns + a.R - x + xx);
-            uint32_t cw[8][2];
+    auto insert = [&](uint32_t key) {
+        if (key < keys[14]) {
 #pragma unroll
-            for (int r = 0; r < 7; ++r) {
-                cw[r][0] = colp[r * wpr];
-                cw[r][1] = colp[r * wpr + 1];
+            for (int m = 0; m < 15; ++m) {
+                const uint32_t lo = min(keys[m], key);
+                key = max(keys[m], key);
+                keys[m] = lo;
             }
-            cw[7][0] = cw[7][1] = 0U;
-            for (int y0 = 0; y0 < ny; y0 += 8) {
-                const uint32_t* rp = colp + (y0 + 7) * wpr;
+        }
+    };
+
+    // The walk over one tile of columns, four rows at a time: body(k, row, s of
+    // row j = 0..3 x columns 2q, 2q + 1, the two (negated) energies, whether
+    // every row j has the candidates in its window), k = 0..3 the row's place
+    // among the four.  Rows that all references have take most of it.
+    const int all0 = max(ylo, y[3] - a.R), all1 = min(yhi, y[0] + a.R);
+    auto tile_walk = [&](int xt, auto&& body) {
+        const int c = xt - rx0 + g + 4 * (q & 1);
+        const uint32_t* bp = s_w + (c & 3) * a.plane + (c >> 2) + (ylo - ry0 + (q >> 1)) * a.wpr;
+        const int* ep = s_e + (ylo - ry0) * a.epitch + xt - rx0 + 2 * q;
+        auto row = [&](auto k, int yy, auto all) {
+            const int2 e = *reinterpret_cast<const int2*>(ep + k * a.epitch);
+            const int h0 = e.x >> 1, h1 = e.y >> 1;
+            const uint32_t f0 = bp[k * a.wpr], f2 = bp[(k + 2) * a.wpr], f4 = bp[(k + 4) * a.wpr], f6 = bp[(k + 6) * a.wpr];
+            int s[4][2];
 #pragma unroll
-                for (int st = 0; st < 8; ++st) {
-                    if (y0 + st < ny) {
-                        cw[(st + 7) & 7][0] = rp[st * wpr];
-                        cw[(st + 7) & 7][1] = rp[st * wpr + 1];
-                        uint32_t d = 0;
+            for (int m = 0; m < 2; ++m) {
+                int d[4];
+                mma_u8(d, af[2 * m][0], af[2 * m + 1][0], af[2 * m][1], af[2 * m + 1][1], f0, f2, h0, h1, h0, h1);
+                mma_u8(d, af[2 * m][2], af[2 * m + 1][2], af[2 * m][3], af[2 * m + 1][3], f4, f6, d[0], d[1], d[2], d[3]);
+                s[2 * m][0] = d[0], s[2 * m][1] = d[1], s[2 * m + 1][0] = d[2], s[2 * m + 1][1] = d[3];
+            }
+            body(k, yy, s, e, all);
+        };
+        using std::integral_constant;
+        for (int yy = ylo; yy <= yhi; yy += 4) {
+            if (yy >= all0 && yy + 3 <= all1) {
+                row(integral_constant<int, 0>{}, yy, std::true_type{});
+                row(integral_constant<int, 1>{}, yy + 1, std::true_type{});
+                row(integral_constant<int, 2>{}, yy + 2, std::true_type{});
+                row(integral_constant<int, 3>{}, yy + 3, std::true_type{});
+            } else {
+                row(integral_constant<int, 0>{}, yy, std::false_type{});
+                if (yy + 1 <= yhi) row(integral_constant<int, 1>{}, yy + 1, std::false_type{});
+                if (yy + 2 <= yhi) row(integral_constant<int, 2>{}, yy + 2, std::false_type{});
+                if (yy + 3 <= yhi) row(integral_constant<int, 3>{}, yy + 3, std::false_type{});
+            }
+            bp += 4 * a.wpr;
+            ep += 4 * a.epitch;
+        }
+    };
+    auto row_in = [&](int yy, int j) { return (unsigned)(yy - y[j] + a.R) <= 2U * a.R; };
+    // whether columns 2q, 2q + 1 of the tile lie in the window of the lane's reference column
+    auto column_in = [&](int xt, int c) {
+        const int xx = xt + 2 * q + c;
+        return xx >= x - a.R && xx <= x + a.R && xx >= 0 && xx <= a.w - 8;
+    };
+
+    if (a.n2 > 1) {
+        // pass 1: a bucket is one residue of columns modulo 8 and of rows modulo
+        // 4, so that good candidates lying together spread over the buckets
+        int best[4][4][2];
 #pragma unroll
-                        for (int r = 0; r < 8; ++r) {
-                            const uint32_t a0 = __vabsdiffu4(rw[2 * r], cw[(st + r) & 7][0]);
-                            d = __dp4a(a0, a0, d);
-                            const uint32_t a1 = __vabsdiffu4(rw[2 * r + 1], cw[(st + r) & 7][1]);
-                            d = __dp4a(a1, a1, d);
-                        }
-                        const int yy = ylo + y0 + st;
-                        if (d <= a.dthr && (xx != x || yy != y)) {
-                            uint32_t key = (d << 11) | (wcol + (uint32_t)((y0 + st) * a.ns));
-                            if (key < keys[14]) {
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-                                for (int m = 0; m < 15; ++m) {
-                                    const uint32_t lo = min(keys[m], key);
-                                    key = max(keys[m], key);
-                                    keys[m] = lo;
-                                }
-                            }
-                        }
+            for (int j = 0; j < 4; ++j) best[k][j][0] = best[k][j][1] = kNone;
+        for (int xt = xs; xt <= xhi; xt += 8) {
+            const int off0 = column_in(xt, 0) ? 0 : kNone, off1 = column_in(xt, 1) ? 0 : kNone;
+            tile_walk(xt, [&](auto k, int yy, const int (&s)[4][2], const int2&, auto all) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool in = all || row_in(yy, j);
+                    best[k][j][0] = __viaddmax_s32(s[j][0], in ? off0 : kNone, best[k][j][0]);
+                    best[k][j][1] = __viaddmax_s32(s[j][1], in ? off1 : kNone, best[k][j][1]);
+                }
+            });
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) s_q[(8 * j + g) * kMatchStride + 8 * k + 2 * q + c] = (uint32_t)best[k][j][c];
+        __syncwarp();
+        {  // lane = reference (row lane / 8, column lane % 8): the 16th largest of its buckets
+            int top[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m) top[m] = kNone;
+            for (int b = 0; b < kMatchQueue; ++b) {
+                int v = (int)s_q[lane * kMatchStride + b];
+#pragma unroll
+                for (int m = 0; m < 16; ++m) {
+                    const int hi = max(top[m], v);
+                    v = min(top[m], v);
+                    top[m] = hi;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) lim[j] = max(lim[j], 2 * __shfl_sync(0xFFFFFFFFU, top[15], 8 * j + g) - 1);
+            s_q[lane * kMatchStride + kMatchQueue] = 0;
+        }
+        __syncwarp();
+        // pass 2
+        const int own = a.R * a.ns + a.R;  // window index of the reference itself
+        int er_own = er[0];                // energy of the lane's reference as the queue's owner (row lane / 8, column lane % 8)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int v = __shfl_sync(0xFFFFFFFFU, er[j], 4 * (lane & 7));
+            if (lane >> 3 == j) er_own = v;
+        }
+        auto drain = [&]() {
+            __syncwarp();
+            uint32_t* mine = s_q + lane * kMatchStride;
+            const int n = (int)mine[kMatchQueue];
+            const int most = __reduce_max_sync(0xFFFFFFFFU, n);
+            for (int i = 0; i < most; ++i) {
+                const uint32_t key = i < n ? mine[i] : 0xFFFFFFFFU;
+                insert((key >> 11) <= a.dthr && (int)(key & 2047U) != own ? key : 0xFFFFFFFFU);
+            }
+            mine[kMatchQueue] = 0;
+            __syncwarp();
+        };
+        bool full = false;
+        // key of candidate (column, row) = key0[j] + row * ns + column - (v << 11)
+        uint32_t key0[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            key0[j] = ((uint32_t)er[j] << 11) + (uint32_t)((a.R - y[j]) * a.ns + a.R - x + 2 * q);
+        const int tiles = (xhi - xs) / 8 + 1;
+        unsigned col0 = 0, col1 = 0;  // bit t: column 2q (2q + 1) of tile t lies in the window
+        for (int t = 0; t < tiles; ++t) {
+            col0 |= column_in(xs + 8 * t, 0) ? 1U << t : 0U;
+            col1 |= column_in(xs + 8 * t, 1) ? 1U << t : 0U;
+        }
+        const int c = xs - rx0 + g + 4 * (q & 1);
+        const uint32_t* brow = s_w + (c & 3) * a.plane + (c >> 2) + (ylo - ry0 + (q >> 1)) * a.wpr;
+        const int* erow = s_e + (ylo - ry0) * a.epitch + xs - rx0 + 2 * q;
+        for (int yy = ylo; yy <= yhi; ++yy, brow += a.wpr, erow += a.epitch) {
+            unsigned rows = 0;  // bits of the rows j with this row in their windows
+#pragma unroll
+            for (int j = 0; j < 4; ++j) rows |= row_in(yy, j) ? 3U << (6 - 2 * j) : 0U;
+#pragma unroll 2
+            for (int t = 0; t < tiles; ++t) {
+                const uint32_t* bp = brow + 2 * t;
+                const int2 e = *reinterpret_cast<const int2*>(erow + 8 * t);
+                const uint32_t f0 = bp[0], f2 = bp[2 * a.wpr], f4 = bp[4 * a.wpr], f6 = bp[6 * a.wpr];
+                int v[4][2];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const uint32_t(&u)[4] = af[2 * m];
+                    const uint32_t(&w)[4] = af[2 * m + 1];
+                    int d[4], p[4];  // twice r.c (two chains of products), minus E
+                    mma_u8(d, u[0], w[0], u[1], w[1], f0, f2, e.x, e.y, e.x, e.y);
+                    mma_u8(p, u[0], w[0], u[1], w[1], f0, f2, d[0], d[1], d[2], d[3]);
+                    mma_u8(d, u[2], w[2], u[3], w[3], f4, f6, p[0], p[1], p[2], p[3]);
+                    mma_u8(p, u[2], w[2], u[3], w[3], f4, f6, d[0], d[1], d[2], d[3]);
+                    v[2 * m][0] = p[0], v[2 * m][1] = p[1], v[2 * m + 1][0] = p[2], v[2 * m + 1][1] = p[3];
+                }
+                unsigned pass = 0;  // bit 7 - (2 j + c): lim - v is negative
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    pass = __funnelshift_l((unsigned)(lim[j] - v[j][0]), pass, 1);
+                    pass = __funnelshift_l((unsigned)(lim[j] - v[j][1]), pass, 1);
+                }
+                pass &= rows & ((col0 >> t & 1U ? 0xAAU : 0U) | (col1 >> t & 1U ? 0x55U : 0U));
+                if (__any_sync(0xFFFFFFFFU, pass != 0)) {
+                    while (pass) {
+                        const int b = __clz(pass) - 24;  // 2 j + c
+                        pass &= ~(128U >> b);
+                        const bool c1 = b & 1;
+                        const int j = b >> 1;
+                        const int v0 = c1 ? v[0][1] : v[0][0], v1 = c1 ? v[1][1] : v[1][0];
+                        const int v2 = c1 ? v[2][1] : v[2][0], v3 = c1 ? v[3][1] : v[3][0];
+                        const int vv = j & 2 ? (j & 1 ? v3 : v2) : (j & 1 ? v1 : v0);
+                        const uint32_t k0 = j & 2 ? (j & 1 ? key0[3] : key0[2]) : (j & 1 ? key0[1] : key0[0]);
+                        uint32_t* mine = s_q + (8 * j + g) * kMatchStride;
+                        const uint32_t at = atomicAdd(mine + kMatchQueue, 1U);
+                        mine[at] = k0 + (uint32_t)(yy * a.ns + xs + 8 * t + c1) - ((uint32_t)vv << 11);
+                        full |= at >= kMatchQueue - 8;
+                    }
+                    if (__any_sync(0xFFFFFFFFU, full)) {  // a tile's row may queue eight more
+                        full = false;
+                        drain();
+                        // only a smaller distance than the 15th best can still enter:
+                        // the walk is in raster order, so an equal one has a larger index
+                        const int bound = keys[14] == 0xFFFFFFFFU ? 2 * kNone : er_own - (int)(keys[14] >> 11);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) lim[j] = max(lim[j], __shfl_sync(0xFFFFFFFFU, bound, 8 * j + g));
                     }
                 }
             }
         }
+        drain();
     }
-    const long long ref = ((long long)img * a.nry + j) * a.nrx + i;
+    // lane = reference: write its list
+    const int ri = wi + (lane & 7), rj = wj + (lane >> 3);
+    if (ri >= a.nrx || rj >= a.nry) return;
+    const int rx = refpos(ri, a.w, a.nstep), ry = row0 + refpos(rj, a.h, a.nstep);
+    const long long ref = ((long long)img * a.nry + rj) * a.nrx + ri;
     uint32_t* out = a.list + ref * 16;
-    out[0] = ((uint32_t)y << 16) | (uint32_t)x;
+    out[0] = ((uint32_t)ry << 16) | (uint32_t)rx;
     int n = 1;
 #pragma unroll
     for (int m = 0; m < 15; ++m) {
         if (m < a.n2 - 1 && keys[m] != 0xFFFFFFFFU) {
             const int widx = (int)(keys[m] & 2047U);
             const int dy = widx / a.ns - a.R, dx = widx % a.ns - a.R;
-            out[1 + m] = ((uint32_t)(y + dy) << 16) | (uint32_t)(x + dx);
+            out[1 + m] = ((uint32_t)(ry + dy) << 16) | (uint32_t)(rx + dx);
             ++n;
         }
     }
@@ -470,11 +699,22 @@ __device__ __forceinline__ void mma1688(float (&c)[4], uint32_t a0, uint32_t a1,
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(b0));
 }
+// The same with a zero addend (one set of zero registers serves every call).
+__device__ __forceinline__ void mma1688_0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};\n"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(b0), "f"(0.0F));
+}
+// a - b, two at a time (the product with -1 is exact).
+__device__ __forceinline__ float2 sub2(const float2& a, const float2& b) {
+    return __ffma2_rn(b, make_float2(-1.0F, -1.0F), a);
+}
 // FP16 hi/lo halves of two floats, packed as (x0, x1) pairs.
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x0, x1);
     const float2 hf = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
+    const float2 r = sub2(make_float2(x0, x1), hf);
+    const __half2 l = __floats2half2_rn(r.x, r.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
@@ -484,8 +724,7 @@ __device__ __forceinline__ void mma_split(float (&c)[4], float a00, float a01, f
     uint32_t h0, l0, h1, l1;
     split2(a00, a01, h0, l0);
     split2(a10, a11, h1, l1);
-    c[0] = c[1] = c[2] = c[3] = 0.0F;
-    mma1688(c, h0, h1, bh);
+    mma1688_0(c, h0, h1, bh);
     mma1688(c, l0, l1, bh);
     mma1688(c, h0, h1, bl);
 }
@@ -498,8 +737,7 @@ __device__ __forceinline__ void mma_split_t(float (&c)[4], const float (&r)[4], 
     l0 = movtrans(l0);
     h1 = movtrans(h1);
     l1 = movtrans(l1);
-    c[0] = c[1] = c[2] = c[3] = 0.0F;
-    mma1688(c, h0, h1, bh);
+    mma1688_0(c, h0, h1, bh);
     mma1688(c, l0, l1, bh);
     mma1688(c, h0, h1, bl);
 }
@@ -517,8 +755,7 @@ __device__ __forceinline__ void mma_prod(float (&c)[4], float a00, float a01, fl
     if (SPLIT) {
         mma_split(c, a00, a01, a10, a11, bh, bl);
     } else {
-        c[0] = c[1] = c[2] = c[3] = 0.0F;
-        mma1688(c, pack2(a00, a01), pack2(a10, a11), bh);
+        mma1688_0(c, pack2(a00, a01), pack2(a10, a11), bh);
     }
 }
 template <bool SPLIT>
@@ -526,8 +763,7 @@ __device__ __forceinline__ void mma_prod_t(float (&c)[4], const float (&r)[4], u
     if (SPLIT) {
         mma_split_t(c, r, bh, bl);
     } else {
-        c[0] = c[1] = c[2] = c[3] = 0.0F;
-        mma1688(c, movtrans(pack2(r[0], r[1])), movtrans(pack2(r[2], r[3])), bh);
+        mma1688_0(c, movtrans(pack2(r[0], r[1])), movtrans(pack2(r[2], r[3])), bh);
     }
 }
 
@@ -552,25 +788,19 @@ __device__ __forceinline__ DctFrags dct_frags(int g, int q) {
 // the forward and the inverse normalisation together.
 template <int S>
 __device__ __forceinline__ void haar_level(float (&H)[8][4]) {
+    // (two coefficients to an instruction)
+    auto butterfly = [](float& lo0, float& lo1, float& hi0, float& hi1) {
+        const float2 lo = make_float2(lo0, lo1), hi = make_float2(hi0, hi1);
+        const float2 sum = __fadd2_rn(lo, hi), dif = sub2(lo, hi);
+        lo0 = sum.x, lo1 = sum.y, hi0 = dif.x, hi1 = dif.y;
+    };
     if (S == 1) {
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float lo = H[t][e], hi = H[t][e + 2];
-                H[t][e] = lo + hi;
-                H[t][e + 2] = lo - hi;
-            }
+        for (int t = 0; t < 8; ++t) butterfly(H[t][0], H[t][1], H[t][2], H[t][3]);
     } else {
         constexpr int D = S / 2;  // distance in t
 #pragma unroll
-        for (int t = 0; t < 8; t += 2 * D)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float lo = H[t][e], hi = H[t + D][e];
-                H[t][e] = lo + hi;
-                H[t + D][e] = lo - hi;
-            }
+        for (int t = 0; t < 8; t += 2 * D) butterfly(H[t][0], H[t][1], H[t + D][0], H[t + D][1]);
     }
 }
 // k of position b > 0 (compile-time after unrolling); position 0 uses log2 N.
@@ -899,7 +1129,20 @@ size_t align256(size_t v) { return (v + 255U) & ~(size_t)255U; }
 size_t filter_smem(const Bm3dPlan& p, int stage) {
     return sizeof(float) * ((size_t)(stage == 2 ? 4 : 3) * p.fw * p.fw + (size_t)kFilterWarps * kWarpBuf + 64);
 }
-size_t match_smem(const Bm3dPlan& p) { return sizeof(uint32_t) * 4 * (size_t)p.mwin * p.mwpr; }
+// The match kernel's region for `tile` x `tile` references: its edge, the word
+// pitches (rows 4 mod 8, copies 8 mod 32, with a spare row and the columns a
+// last tile of eight may reach over), the energies' pitch, and the bytes.
+size_t match_layout(Bm3dPlan& p, int tile) {
+    p.mtile = tile;
+    p.mwin = (tile - 1) * p.nstep + 2 * p.R + 8;
+    const int wpr = (p.mwin + 11) / 4 + 1;
+    p.mwpr = wpr + ((4 - wpr) % 8 + 8) % 8;
+    const int plane = (p.mwin + 1) * p.mwpr;
+    p.mplane = plane + ((8 - plane) % 32 + 32) % 32;
+    p.mepitch = (p.mwin + 2) & ~1;
+    return sizeof(uint32_t) *
+           (4 * (size_t)p.mplane + (size_t)p.mepitch * (p.mwin - 7) + (size_t)(tile * tile) * kMatchStride);
+}
 // Row pitch of the tensor-core form's footprint planes: at least fw and 4 mod
 // 32 (column loads of eight columns x two rows, and atomics of eight rows x
 // four columns, fall in 32 different banks).
@@ -961,8 +1204,9 @@ int bm3d_plan(const cpipe_Bm3dSpecParams* p, int w, int h, Bm3dPlan* out, int ba
     q.phases = (span + 2 * q.R + 8 + span - 1) / span;
     q.ntx = (q.nrx + kRefTile - 1) / kRefTile;
     q.nty = (q.nry + kRefTile - 1) / kRefTile;
-    q.mwin = (kMatchTile - 1) * q.nstep + 2 * q.R + 8;
-    q.mwpr = (q.mwin + 3) / 4 + 1;
+    // 16 x 16 references a CTA share a region best; the largest windows and steps need 8 x 8
+    q.match_bytes = match_layout(q, 16);
+    if (q.match_bytes > 227 * 1024) q.match_bytes = match_layout(q, 8);
     const size_t npx = (size_t)w * h * batch, nref = (size_t)q.nrx * q.nry * batch;
     size_t o = 0;
     q.off_yuv = o;
@@ -984,11 +1228,9 @@ int bm3d_plan(const cpipe_Bm3dSpecParams* p, int w, int h, Bm3dPlan* out, int ba
 cudaError_t bm3d_setup(const Bm3dPlan& p) {
     if (p.copy) return cudaSuccess;
     static const size_t kSmemOptIn = 227 * 1024;
-    const size_t ms = match_smem(p), fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
+    const size_t ms = p.match_bytes, fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
     if (ms > kSmemOptIn || fs2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(bm3d_match_kernel<kMatchWprStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bm3d_match_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms);
+    cudaError_t e = cudaFuncSetAttribute(bm3d_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(bm3d_filter_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs1);
     if (e == cudaSuccess)
@@ -1022,15 +1264,16 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     const long long npx = (long long)p.w * p.h * p.batch;
     cudaError_t e;
     if (setup && (e = bm3d_setup(p)) != cudaSuccess) return e;
-    const size_t ms = match_smem(p), fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
+    const size_t fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
     const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
 
     const dim3 pgrid((p.w + 255) / 256, p.h * p.batch);
     if (f16) bm3d_prep_kernel<__half><<<pgrid, 256, 0, st>>>(in, yuv, q, npx, gate);
     else bm3d_prep_kernel<float><<<pgrid, 256, 0, st>>>(in, yuv, q, npx, gate);
 
-    MatchArgs ma{p.w, p.h, p.nrx, p.nry, p.nstep, p.R, p.ns, p.n2, p.mwpr, p.mwin, p.dthr[0], q, list, cnt, gate};
-    const dim3 mgrid((p.nrx + kMatchTile - 1) / kMatchTile, (p.nry + kMatchTile - 1) / kMatchTile, p.batch);
+    MatchArgs ma{p.w,    p.h,      p.nrx,     p.nry, p.nstep, p.R, p.ns, p.n2, p.mtile,
+                 p.mwpr, p.mplane, p.mepitch, p.dthr[0], q, list, cnt, gate};
+    const dim3 mgrid((p.nrx + p.mtile - 1) / p.mtile, (p.nry + p.mtile - 1) / p.mtile, p.batch);
     FilterArgs fa{};
     fa.w = p.w;
     fa.h = p.h;
@@ -1062,8 +1305,7 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     for (int stage = 1; stage <= p.stages; ++stage) {
         bm3d_zero_kernel<<<kSmCount * 8, 256, 0, st>>>(acc, 6 * npx, gate);
         ma.dthr = p.dthr[stage - 1];
-        if (p.mwpr == kMatchWprStd) bm3d_match_kernel<kMatchWprStd><<<mgrid, kMatchTile * kMatchTile, ms, st>>>(ma);
-        else bm3d_match_kernel<0><<<mgrid, kMatchTile * kMatchTile, ms, st>>>(ma);
+        bm3d_match_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
         if (p.tensor) {
             if (p.split) {
                 if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);

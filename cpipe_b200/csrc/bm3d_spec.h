@@ -23,7 +23,9 @@ struct Bm3dPlan {
     int fw = 0;            // filter footprint edge bound (pixels)
     int phases = 0;        // filter launch phases per axis
     int ntx = 0, nty = 0;  // filter tiles (8x8 reference blocks each)
-    int mwin = 0, mwpr = 0;  // match tile region edge bound, words per smem row
+    // match kernel: references per CTA edge, region edge bound, pitches in words, shared memory
+    int mtile = 0, mwin = 0, mwpr = 0, mplane = 0, mepitch = 0;
+    size_t match_bytes = 0;
     bool copy = false;       // image below 8x8 or sigma <= 0: output = input
     bool tensor = true;      // transforms on the tensor cores or FP32 CUDA cores
     bool split = true;       // tensor cores: FP16 hi/lo split products (else single FP16 products)

@@ -66,6 +66,22 @@ def test_bm3d_spec_matches_fp64_oracle(cuda_device, h, w, sigma, kw):
     compare(got.astype(np.float32), want, f"{w}x{h} sigma {sigma} {kw}")
 
 
+# the largest windows and steps (8x8 references a CTA instead of 16x16), windows of one tile of columns, a posterised
+# scene whose distances tie so often that a reference's candidate queue is sorted in early
+@pytest.mark.parametrize("h,w,kw,levels", [(120, 200, dict(ns=45, nstep=8), 0), (97, 131, dict(ns=45, nstep=2), 0),
+                                           (33, 260, dict(ns=5, nstep=3), 0), (90, 121, dict(ns=1), 0),
+                                           (72, 100, dict(tau_match1=16000.0, tau_match2=16000.0), 3),
+                                           (64, 64, dict(tau_match1=0.0, tau_match2=0.0), 2)])
+def test_bm3d_spec_windows_and_ties(cuda_device, h, w, kw, levels):
+    clean = clean_rgb(h + w, h, w)
+    if levels:
+        clean = np.round(clean * levels) / levels
+    x = noisy_rgba(clean, 0.0 if levels else 0.03, h)
+    blob = blobs.bm3d_spec(0.03, **kw)
+    want = oracle.bm3d_spec(x.astype(np.float32), blob)
+    compare(gpu_bm3d(x, blob).astype(np.float32), want, f"{w}x{h} {kw} levels {levels}")
+
+
 def test_bm3d_spec_f32_buffers(cuda_device):
     clean = clean_rgb(5, 72, 88)
     x = noisy_rgba(clean, 0.03, 5, dtype=np.float32)
