@@ -52,9 +52,19 @@ struct RawLoader {
     }
 };
 
-template <int ALGO, class TOut>
+template <int ALGO, class TOut, int TW, int TH>
 __global__ void __launch_bounds__(256) raw_to_rgba_kernel(Img raw, Img out, RawParams p) {
-    demosaic_tile<ALGO, TOut>(RawLoader{raw, &p}, raw.w, raw.h, out, p.cfa);
+    demosaic_tile<ALGO, TOut, TW, TH>(RawLoader{raw, &p}, raw.w, raw.h, out, p.cfa);
+}
+template <int ALGO, class TOut>
+void launch_raw_to_rgba(const Img& raw, const Img& out, const RawParams& p, cudaStream_t st) {
+    const dim3 g((unsigned)((raw.w + kDmTW - 1) / kDmTW), (unsigned)((raw.h + kDmTH - 1) / kDmTH));
+    if ((long long)g.x * g.y < kSmCount) {
+        const dim3 gs((unsigned)((raw.w + kDmTWs - 1) / kDmTWs), (unsigned)((raw.h + kDmTHs - 1) / kDmTHs));
+        raw_to_rgba_kernel<ALGO, TOut, kDmTWs, kDmTHs><<<gs, kDmThreads, 0, st>>>(raw, out, p);
+    } else {
+        raw_to_rgba_kernel<ALGO, TOut, kDmTW, kDmTH><<<g, kDmThreads, 0, st>>>(raw, out, p);
+    }
 }
 
 // ------------------------------------------------------------------ K2
@@ -113,20 +123,33 @@ __global__ void __launch_bounds__(128) warp_wb_cm_kernel(Img in, Img out, WarpDe
 }
 
 // ------------------------------------------------------------------ K3
-// Tile TW x TH; R = guided box radius (0: no guided node, 1: 3x3, 2: 5x5).
-// Shared-memory planes (3 colour channels each, float: every value stored is
-// either an f16 node output or an f32 intermediate, so no precision is lost),
-// indexed by unclamped coordinate relative to the tile origin:
-//   s_bm : BM3D output at clamp(coord), coords [x0-2R, x0+TW+2R)
-//   s_a/s_b : guided a, b at coords [x0-R, x0+TW+R)
-//   s_gf : guided output for the tile (needed whole for the wavelet 2x2 blocks)
+// Tile kCTW x kCTH; R = guided box radius (0: no guided node, 1: 3x3, 2: 5x5).
+// A thread owns one aligned 2x2 block of the tile for everything that is defined
+// per block or pixel (wavelet, tone, LUT).  Without the guided node that is all:
+// the blend's block is the same one, and nothing goes through shared memory.
+// With it, shared-memory planes (3 colour channels each, float: every value
+// stored is either an f16 node output or an f32 intermediate, so no precision
+// is lost), indexed by unclamped coordinate relative to the tile origin:
+//   s_bm : BM3D output at clamp(coord), coords [x0-2R, x0+TW+2R); the guided
+//          output replaces a tile pixel's value in place (only its own thread
+//          still reads it)
+//   s_ab : guided (a, b) at coords [x0-R, x0+TW+R)
 // BM3D is evaluated per 2x2 block of the extent (x0 and 2R are even, so the
 // extent is made of whole blocks): an interior block reads its four input
 // pixels with two 16-byte loads and yields four outputs; a block that overlaps
 // the frame border evaluates each cell at its clamped coordinate.
-// Box sums keep the generator's row-major left-to-right order; a thread loads
-// one (G+2R) x (2R+1) window into registers and produces G outputs from it.
-constexpr int kCTW = 64, kCTH = 16, kCG = 4;
+// Box sums keep the generator's row-major left-to-right order; a thread sums
+// kCG x kCGR outputs at once while it walks down the rows of their windows (the
+// running sums and one row in registers), so a row's values are read from shared
+// memory once, 16 bytes at a time, for all the sums they enter.  kCGR = 4, and
+// tone and LUT unrolled over the whole block, took a fifth fewer instructions
+// than one column of four rows but ran slower: the code outgrew the instruction
+// cache (583 us at 12 MP).
+constexpr int kCTW = 64, kCTH = 16, kCG = 4, kCGR = 2;
+// A frame of fewer tiles than SMs is bound by one tile's latency: tiles a
+// quarter the size spread it over four times the SMs, and every stage is one
+// pass of the CTA's threads.
+constexpr int kCTWs = 32, kCTHs = 8;
 
 struct ToneParams {
     int has_wavelet;
@@ -141,16 +164,16 @@ struct ToneParams {
     int has_lut;
 };
 
-template <int R>
+template <int R, int TW, int TH>
 struct ToneGeom {
     static constexpr int H = 2 * R;
-    static constexpr int CW = kCTW + 2 * H, CH = kCTH + 2 * H;  // bm3d extent
-    static constexpr int CP = CW + 1;                           // padded row pitch
-    static constexpr int AW = kCTW + 2 * R, AH = kCTH + 2 * R;  // a / b extent
-    static constexpr int AP = AW + 1;
-    static constexpr int AB = R > 0 ? AP * AH : 0;
-    static constexpr int D = 2 * R + 1;
-    static constexpr size_t bytes() { return sizeof(float) * (size_t)(3 * CP * CH + 2 * 3 * AB + 3 * kCTW * kCTH); }
+    static constexpr int CW = TW + 2 * H, CH = TH + 2 * H;  // bm3d extent
+    static constexpr int AW = TW + 2 * R, AH = TH + 2 * R;  // a / b extent
+    static constexpr int GX = (AW + kCG - 1) / kCG, GY = (AH + kCGR - 1) / kCGR;  // a / b items
+    static constexpr int CP = kCG * GX + 4, CHP = kCGR * GY + 2 * R;  // pitch and rows that whole items read
+    static constexpr int AP = TW + 4;                                // (a, b) pitch, in pairs
+    static_assert(CP >= CW && CHP >= CH && AP >= AW && CP % 4 == 0, "tile geometry");
+    static constexpr size_t bytes() { return R == 0 ? 0 : sizeof(float) * (size_t)(3 * CP * CHP + 2 * 3 * AP * AH); }
 };
 
 template <class T>
@@ -178,158 +201,241 @@ __device__ __forceinline__ void load_pair<float>(const Img& in, int x, int y, Rg
     *b = load_rgba(px<const float>(in, x + 1, y));
 }
 
-// One kCTW x kCTH output tile at (x0, y0); smem_f: denoise_tone_smem bytes.
-template <class T, bool F16, int R>
+
+// v at pixel (u + k % 2, v + k / 2) of an aligned 2x2 block -> the block blended
+// toward its mean (bm3d_step1_generator.cpp:42-56), in the node's rounding.
+template <bool F16>
+__device__ __forceinline__ void blend_block(const Rgba (&q)[4], float s, Rgba (&o)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        o[k] = Rgba{rnd<F16>(bm3d_blend(q[k].r, q[0].r, q[1].r, q[2].r, q[3].r, s)),
+                    rnd<F16>(bm3d_blend(q[k].g, q[0].g, q[1].g, q[2].g, q[3].g, s)),
+                    rnd<F16>(bm3d_blend(q[k].b, q[0].b, q[1].b, q[2].b, q[3].b, s)), q[k].a};
+}
+// The four pixels of the block at (u, v), those past the frame's right or lower edge clamped.
+template <class T>
+__device__ __forceinline__ void load_block(const Img& in, int u, int v, Rgba (&q)[4]) {
+    if (u + 1 < in.w && v + 1 < in.h) {
+        load_pair<T>(in, u, v, &q[0], &q[1]);
+        load_pair<T>(in, u, v + 1, &q[2], &q[3]);
+    } else {
+        const int u1 = min(u + 1, in.w - 1), v1 = min(v + 1, in.h - 1);
+        q[0] = load_rgba(px<const T>(in, u, v));
+        q[1] = load_rgba(px<const T>(in, u1, v));
+        q[2] = load_rgba(px<const T>(in, u, v1));
+        q[3] = load_rgba(px<const T>(in, u1, v1));
+    }
+}
+__device__ __forceinline__ void store_pair(const Img& out, __half* p, const Rgba& a, const Rgba& b, bool two) {
+    if (two && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && out.pix_stride == 4) {
+        __align__(16) __half2 h[4] = {__floats2half2_rn(a.r, a.g), __floats2half2_rn(a.b, a.a),
+                                      __floats2half2_rn(b.r, b.g), __floats2half2_rn(b.b, b.a)};
+        *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+        return;
+    }
+    store_rgba(p, a);
+    if (two) store_rgba(p + out.pix_stride, b);
+}
+__device__ __forceinline__ void store_pair(const Img& out, float* p, const Rgba& a, const Rgba& b, bool two) {
+    store_rgba(p, a);
+    if (two) store_rgba(p + out.pix_stride, b);
+}
+// Wavelet, tone and LUT on the aligned 2x2 block at (x, y): q its (guided)
+// values, alpha included; cells outside the frame hold their clamped neighbour.
+template <class T, bool F16>
+__device__ __forceinline__ void tone_block(const Img& out, const ToneParams& p, int x, int y, Rgba (&q)[4]) {
+    if (p.has_wavelet) {
+        wavelet_block(q, p.wavelet_th);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = Rgba{rnd<F16>(q[k].r), rnd<F16>(q[k].g), rnd<F16>(q[k].b), rnd<F16>(q[k].a)};
+    }
+    const bool two = x + 1 < out.w;
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {  // (rows in turn: half the code)
+        if (y + r >= out.h) break;
+        Rgba v[2] = {r ? q[2] : q[0], r ? q[3] : q[1]};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (p.tone_op == 0) v[k] = filmic_px(v[k], p.filmic);
+            else if (p.tone_op == 1) v[k] = Rgba{aces_fit(v[k].r), aces_fit(v[k].g), aces_fit(v[k].b), v[k].a};
+            else v[k] = Rgba{reinhard_px(v[k].r, p.reinhard_wp2), reinhard_px(v[k].g, p.reinhard_wp2), reinhard_px(v[k].b, p.reinhard_wp2), v[k].a};
+            if (p.has_lut) {
+                v[k] = Rgba{rnd<F16>(v[k].r), rnd<F16>(v[k].g), rnd<F16>(v[k].b), v[k].a};
+                v[k] = lut_px(v[k], p.lut, p.lut_size, p.lut_interp);
+            }
+        }
+        store_pair(out, px<T>(out, x, y + r), v[0], v[1], two);
+    }
+}
+
+// One row of a window walk: w the row's values, its row number r among the rows
+// of kCGR outputs; every running sum the row belongs to takes its D values in order.
+template <int D>
+__device__ __forceinline__ void box_row(float2 (&sum)[kCGR][kCG], const float2 (&w)[kCG + D - 1], int r) {
+#pragma unroll
+    for (int ky = 0; ky < kCGR; ++ky) {
+        const int dy = r - ky;
+        if (dy < 0 || dy >= D) continue;
+#pragma unroll
+        for (int kx = 0; kx < kCG; ++kx)
+#pragma unroll
+            for (int dx = 0; dx < D; ++dx)
+                sum[ky][kx] = dy == 0 && dx == 0 ? w[kx] : __fadd2_rn(sum[ky][kx], w[kx + dx]);
+    }
+}
+
+// One TW x TH output tile at (x0, y0); smem_f: ToneGeom::bytes().
+template <class T, bool F16, int R, int TW = kCTW, int TH = kCTH>
 __device__ __forceinline__ void denoise_tone_tile(const Img& in, const Img& out, const ToneParams& p, int x0, int y0,
                                                   float* smem_f) {
-    using Gm = ToneGeom<R>;
-    constexpr int H = Gm::H, CW = Gm::CW, CH = Gm::CH, CP = Gm::CP, AW = Gm::AW, AH = Gm::AH, AP = Gm::AP;
-    constexpr int AB = Gm::AB, D = Gm::D;
-    float* s_bm = smem_f;
-    float* s_a = s_bm + 3 * CP * CH;
-    float* s_b = s_a + 3 * AB;
-    float* s_gf = s_b + 3 * AB;
-    const int cx0 = x0 - H, cy0 = y0 - H;
+    using Gm = ToneGeom<R, TW, TH>;
     const float s = p.bm3d_strength;
-    // 1) BM3D parity form (bm3d_step1_generator.cpp:42-56) per 2x2 block of the extent
-    for (int item = threadIdx.x; item < (CW / 2) * (CH / 2); item += blockDim.x) {
-        const int by2 = item / (CW / 2), bx2 = item - by2 * (CW / 2);
-        const int u = cx0 + 2 * bx2, v = cy0 + 2 * by2;  // unclamped block origin
-        const int l = (2 * by2) * CP + 2 * bx2;
-        if (u >= 0 && u + 1 < in.w && v >= 0 && v + 1 < in.h) {
-            Rgba q[4];
-            load_pair<T>(in, u, v, &q[0], &q[1]);
-            load_pair<T>(in, u, v + 1, &q[2], &q[3]);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int o = l + (k >> 1) * CP + (k & 1);
-                s_bm[o] = rnd<F16>(bm3d_blend(q[k].r, q[0].r, q[1].r, q[2].r, q[3].r, s));
-                s_bm[CP * CH + o] = rnd<F16>(bm3d_blend(q[k].g, q[0].g, q[1].g, q[2].g, q[3].g, s));
-                s_bm[2 * CP * CH + o] = rnd<F16>(bm3d_blend(q[k].b, q[0].b, q[1].b, q[2].b, q[3].b, s));
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int xc = clampi(u + (k & 1), 0, in.w - 1), yc = clampi(v + (k >> 1), 0, in.h - 1);
-                const int bx = xc & ~1, by = yc & ~1;
-                const int bx1 = min(bx + 1, in.w - 1), by1 = min(by + 1, in.h - 1);
-                const Rgba q0 = load_rgba(px<const T>(in, bx, by)), q1 = load_rgba(px<const T>(in, bx1, by));
-                const Rgba q2 = load_rgba(px<const T>(in, bx, by1)), q3 = load_rgba(px<const T>(in, bx1, by1));
-                const Rgba c = load_rgba(px<const T>(in, xc, yc));
-                const int o = l + (k >> 1) * CP + (k & 1);
-                s_bm[o] = rnd<F16>(bm3d_blend(c.r, q0.r, q1.r, q2.r, q3.r, s));
-                s_bm[CP * CH + o] = rnd<F16>(bm3d_blend(c.g, q0.g, q1.g, q2.g, q3.g, s));
-                s_bm[2 * CP * CH + o] = rnd<F16>(bm3d_blend(c.b, q0.b, q1.b, q2.b, q3.b, s));
-            }
-        }
-    }
-    __syncthreads();
-    constexpr float N = (float)(D * D);
-    const ConstDiv cN{N, (float)(1.0 / (double)(D * D))};  // IEEE x / N (const_div)
-    if (R == 0) {  // no guided node: the wavelet reads the BM3D output
-        for (int i = threadIdx.x; i < 3 * kCTW * kCTH; i += blockDim.x) {
-            const int c = i / (kCTW * kCTH);
-            const int j = i - c * kCTW * kCTH;
-            const int ty = j / kCTW, tx = j - ty * kCTW;
-            s_gf[i] = s_bm[c * CP * CH + ty * CP + tx];
-        }
+    if constexpr (R == 0) {
+        const int x = x0 + 2 * (int)(threadIdx.x % (TW / 2)), y = y0 + 2 * (int)(threadIdx.x / (TW / 2));
+        if (x >= out.w || y >= out.h) return;
+        Rgba q[4], v[4];
+        load_block<T>(in, x, y, q);
+        blend_block<F16>(q, s, v);
+        tone_block<T, F16>(out, p, x, y, v);
     } else {
-        // 2) guided a, b (guided_filter_generator.cpp:60-76) at unclamped
-        //    coordinates [x0-R, x0+TW+R), kCG rows per thread
-        constexpr int AG = (AH + kCG - 1) / kCG;
-        for (int item = threadIdx.x; item < 3 * AW * AG; item += blockDim.x) {
-            const int c = item / (AW * AG);
-            const int rem = item - c * AW * AG;
-            const int g = rem / AW, tx = rem - g * AW;
-            const int ty0 = g * kCG;
-            const float* V = s_bm + c * CP * CH + ty0 * CP + tx;  // window origin of output (ty0, tx)
-            float2 win[kCG + 2 * R][D];  // (value, value^2)
+        constexpr int H = Gm::H, CW = Gm::CW, CH = Gm::CH, CP = Gm::CP, AW = Gm::AW, AH = Gm::AH, AP = Gm::AP;
+        constexpr int D = 2 * R + 1, CPL = CP * Gm::CHP, APL = AP * AH;  // plane sizes
+        float* s_bm = smem_f;
+        float2* s_ab = reinterpret_cast<float2*>(s_bm + 3 * CPL);
+        const int cx0 = x0 - H, cy0 = y0 - H;
+        // 1) BM3D parity form per 2x2 block of the extent
+        for (int item = threadIdx.x; item < (CW / 2) * (CH / 2); item += blockDim.x) {
+            const int by2 = item / (CW / 2), bx2 = item - by2 * (CW / 2);
+            const int u = cx0 + 2 * bx2, v = cy0 + 2 * by2;  // unclamped block origin
+            const int l = (2 * by2) * CP + 2 * bx2;
+            Rgba o[4];
+            if (u >= 0 && u + 1 < in.w && v >= 0 && v + 1 < in.h) {
+                Rgba q[4];
+                load_pair<T>(in, u, v, &q[0], &q[1]);
+                load_pair<T>(in, u, v + 1, &q[2], &q[3]);
+                blend_block<F16>(q, s, o);
+            } else {
 #pragma unroll
-            for (int r = 0; r < kCG + 2 * R; ++r)
-#pragma unroll
-                for (int dx = 0; dx < D; ++dx) {
-                    const float t = (ty0 + r < CH) ? V[r * CP + dx] : 0.0F;
-                    win[r][dx] = make_float2(t, t * t);
+                for (int k = 0; k < 4; ++k) {
+                    const int xc = clampi(u + (k & 1), 0, in.w - 1), yc = clampi(v + (k >> 1), 0, in.h - 1);
+                    Rgba q[4], b[4];
+                    load_block<T>(in, xc & ~1, yc & ~1, q);
+                    blend_block<F16>(q, s, b);
+                    const int c = (yc & 1) * 2 + (xc & 1);
+                    o[k] = c & 2 ? (c & 1 ? b[3] : b[2]) : (c & 1 ? b[1] : b[0]);
                 }
+            }
 #pragma unroll
-            for (int k = 0; k < kCG; ++k) {
-                if (ty0 + k >= AH) break;
-                const float2 sums = box_chain2<D>(win, k);
-                const float m = const_div(sums.x, cN), corr = const_div(sums.y, cN);
-                const float var = max0(corr - (m * m));
-                const float a = var / (var + p.eps);
-                const int j = c * AB + (ty0 + k) * AP + tx;
-                s_a[j] = a;
-                s_b[j] = m - (a * m);
+            for (int r = 0; r < 2; ++r) {
+                *reinterpret_cast<float2*>(s_bm + l + r * CP) = make_float2(o[2 * r].r, o[2 * r + 1].r);
+                *reinterpret_cast<float2*>(s_bm + CPL + l + r * CP) = make_float2(o[2 * r].g, o[2 * r + 1].g);
+                *reinterpret_cast<float2*>(s_bm + 2 * CPL + l + r * CP) = make_float2(o[2 * r].b, o[2 * r + 1].b);
+            }
+        }
+        __syncthreads();
+        constexpr float N = (float)(D * D);
+        const ConstDiv cN{N, (float)(1.0 / (double)(D * D))};  // IEEE x / N (const_div)
+        // 2) guided a, b (guided_filter_generator.cpp:60-76) at unclamped
+        //    coordinates [x0-R, x0+TW+R)
+        for (int item = threadIdx.x; item < 3 * Gm::GX * Gm::GY; item += blockDim.x) {
+            const int c = item / (Gm::GX * Gm::GY), rem = item - c * (Gm::GX * Gm::GY);
+            const int gy = rem / Gm::GX, tx = kCG * (rem - gy * Gm::GX), ty = kCGR * gy;
+            const float* V = s_bm + c * CPL + ty * CP + tx;  // window origin of output (tx, ty)
+            float2 sum[kCGR][kCG];                            // (value, value^2)
+#pragma unroll
+            for (int r = 0; r < kCGR + D - 1; ++r) {
+                const float4 v0 = *reinterpret_cast<const float4*>(V + r * CP);
+                const float4 v1 = *reinterpret_cast<const float4*>(V + r * CP + 4);
+                const float t[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                float2 w[kCG + D - 1];
+#pragma unroll
+                for (int i = 0; i < kCG + D - 1; ++i) w[i] = make_float2(t[i], t[i] * t[i]);
+                box_row<D>(sum, w, r);
+            }
+#pragma unroll
+            for (int ky = 0; ky < kCGR; ++ky) {
+                if (ty + ky >= AH) break;
+#pragma unroll
+                for (int kx = 0; kx < kCG; ++kx) {
+                    const float2 mc = const_div2(sum[ky][kx], cN);
+                    const float m = mc.x, corr = mc.y;
+                    const float var = max0(corr - (m * m));
+                    const float a = var / (var + p.eps);
+                    if (tx + kx < AW) s_ab[c * APL + (ty + ky) * AP + tx + kx] = make_float2(a, m - (a * m));
+                }
             }
         }
         __syncthreads();
         // 3) guided output for the tile: mean(a) * v + mean(b)
-        constexpr int TG = kCTH / kCG;
-        for (int item = threadIdx.x; item < 3 * kCTW * TG; item += blockDim.x) {
-            const int c = item / (kCTW * TG);
-            const int rem = item - c * kCTW * TG;
-            const int g = rem / kCTW, tx = rem - g * kCTW;
-            const int ty0 = g * kCG;
-            float2 win[kCG + 2 * R][D];  // (a, b)
-            const float* A = s_a + c * AB + ty0 * AP + tx;
-            const float* B = s_b + c * AB + ty0 * AP + tx;
+        for (int item = threadIdx.x; item < 3 * (TW / kCG) * (TH / kCGR); item += blockDim.x) {
+            const int c = item / ((TW / kCG) * (TH / kCGR)), rem = item - c * ((TW / kCG) * (TH / kCGR));
+            const int tx = kCG * (rem % (TW / kCG)), ty = kCGR * (rem / (TW / kCG));
+            const float2* AB = s_ab + c * APL + ty * AP + tx;
+            float2 sum[kCGR][kCG];
 #pragma unroll
-            for (int r = 0; r < kCG + 2 * R; ++r)
+            for (int r = 0; r < kCGR + D - 1; ++r) {
+                float2 w[8];
 #pragma unroll
-                for (int dx = 0; dx < D; ++dx) win[r][dx] = make_float2(A[r * AP + dx], B[r * AP + dx]);
+                for (int i = 0; i < 8; i += 2) {
+                    if (i >= kCG + D - 1) continue;
+                    const float4 t = *reinterpret_cast<const float4*>(AB + r * AP + i);
+                    w[i] = make_float2(t.x, t.y);
+                    w[i + 1] = make_float2(t.z, t.w);
+                }
+                float2 ww[kCG + D - 1];
 #pragma unroll
-            for (int k = 0; k < kCG; ++k) {
-                const int ty = ty0 + k;
-                const float2 sab = box_chain2<D>(win, k);
-                const float v = s_bm[c * CP * CH + (ty + H) * CP + (tx + H)];
-                s_gf[c * kCTW * kCTH + ty * kCTW + tx] = rnd<F16>(max0((const_div(sab.x, cN) * v) + const_div(sab.y, cN)));
+                for (int i = 0; i < kCG + D - 1; ++i) ww[i] = w[i];
+                box_row<D>(sum, ww, r);
             }
+            float* V = s_bm + c * CPL + (ty + H) * CP + tx + H;
+#pragma unroll
+            for (int ky = 0; ky < kCGR; ++ky)
+#pragma unroll
+                for (int kx = 0; kx < kCG; ++kx) {
+                    const float v = V[ky * CP + kx];
+                    const float2 mab = const_div2(sum[ky][kx], cN);
+                    V[ky * CP + kx] = rnd<F16>(max0((mab.x * v) + mab.y));
+                }
         }
-    }
-    __syncthreads();
-    // 4) wavelet on the aligned 2x2 block, filmic, LUT; one thread per pixel
-    for (int j = threadIdx.x; j < kCTW * kCTH; j += blockDim.x) {
-        const int ty = j / kCTW, tx = j - ty * kCTW;
+        __syncthreads();
+        // 4) wavelet, tone, LUT
+        const int tx = 2 * (int)(threadIdx.x % (TW / 2)), ty = 2 * (int)(threadIdx.x / (TW / 2));
         const int x = x0 + tx, y = y0 + ty;
-        if (x >= out.w || y >= out.h) continue;
-        const int bx = x & ~1, by = y & ~1;
-        const int xs0 = bx - x0, xs1 = min(bx + 1, out.w - 1) - x0;
-        const int ys0 = by - y0, ys1 = min(by + 1, out.h - 1) - y0;
+        if (ty >= TH || x >= out.w || y >= out.h) return;
         Rgba q[4];
+        load_block<T>(in, x, y, q);  // for alpha, which runs through unchanged except the wavelet's max(0, .)
+        const float* g = s_bm + (ty + H) * CP + tx + H;
+        const bool two = x + 1 < out.w, low = y + 1 < out.h;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int l = ((k >> 1) ? ys1 : ys0) * kCTW + ((k & 1) ? xs1 : xs0);
-            q[k] = Rgba{s_gf[l], s_gf[kCTW * kCTH + l], s_gf[2 * kCTW * kCTH + l], 0.0F};
+            const int l = ((k >> 1) && low ? CP : 0) + ((k & 1) && two ? 1 : 0);
+            q[k].r = g[l], q[k].g = g[CPL + l], q[k].b = g[2 * CPL + l];
         }
-        // alpha runs through unchanged except the wavelet's max(0, .)
-        const int ox = x & 1, oy = y & 1;
-        const Rgba own = oy ? (ox ? q[3] : q[2]) : (ox ? q[1] : q[0]);
-        Rgba v{own.r, own.g, own.b, load_rgba(px<const T>(in, x, y)).a};
-        if (p.has_wavelet) {
-            v = wavelet_px(q, v, ox, oy, p.wavelet_th);
-            v = Rgba{rnd<F16>(v.r), rnd<F16>(v.g), rnd<F16>(v.b), rnd<F16>(v.a)};
-        }
-        if (p.tone_op == 0) v = filmic_px(v, p.filmic);
-        else if (p.tone_op == 1) v = Rgba{aces_fit(v.r), aces_fit(v.g), aces_fit(v.b), v.a};
-        else v = Rgba{reinhard_px(v.r, p.reinhard_wp2), reinhard_px(v.g, p.reinhard_wp2), reinhard_px(v.b, p.reinhard_wp2), v.a};
-        if (p.has_lut) {
-            v = Rgba{rnd<F16>(v.r), rnd<F16>(v.g), rnd<F16>(v.b), v.a};
-            v = lut_px(v, p.lut, p.lut_size, p.lut_interp);
-        }
-        store_rgba(px<T>(out, x, y), v);
+        tone_block<T, F16>(out, p, x, y, q);
     }
 }
 
-template <class T, bool F16, int R>
-__global__ void __launch_bounds__(256, 3) denoise_tone_kernel(Img in, Img out, ToneParams p) {
+// Threads of a tile's CTA (without the guided node one per 2x2 block), and the
+// CTAs per SM its registers are held to: 64 registers a thread measured best (12
+// MP, R = 2: 448 us against 463 with 80; R = 0: 149 against 165, and 156 with 40).
+constexpr int tone_threads(int r, int tw, int th) { return r == 0 ? tw * th / 4 : 256; }
+template <class T, bool F16, int R, int TW, int TH>
+__global__ void __launch_bounds__(tone_threads(R, TW, TH), 1024 / tone_threads(R, TW, TH))
+    denoise_tone_kernel(Img in, Img out, ToneParams p) {
     extern __shared__ __align__(16) float smem_f[];
-    denoise_tone_tile<T, F16, R>(in, out, p, (int)blockIdx.x * kCTW, (int)blockIdx.y * kCTH, smem_f);
+    denoise_tone_tile<T, F16, R, TW, TH>(in, out, p, (int)blockIdx.x * TW, (int)blockIdx.y * TH, smem_f);
 }
-
+template <class T, bool F16, int R, int TW, int TH>
+void launch_tone_tiles(const Img& in, const Img& out, const ToneParams& p, cudaStream_t st) {
+    const dim3 grid((unsigned)((in.w + TW - 1) / TW), (unsigned)((in.h + TH - 1) / TH));
+    denoise_tone_kernel<T, F16, R, TW, TH>
+        <<<grid, tone_threads(R, TW, TH), ToneGeom<R, TW, TH>::bytes(), st>>>(in, out, p);
+}
 template <class T, bool F16, int R>
-size_t denoise_tone_smem() {
-    return ToneGeom<R>::bytes();
+void launch_tone(const Img& in, const Img& out, const ToneParams& p, cudaStream_t st) {
+    const long long tiles = (long long)((in.w + kCTW - 1) / kCTW) * ((in.h + kCTH - 1) / kCTH);
+    if (tiles < kSmCount) launch_tone_tiles<T, F16, R, kCTWs, kCTHs>(in, out, p, st);
+    else launch_tone_tiles<T, F16, R, kCTW, kCTH>(in, out, p, st);
 }
 
 }  // namespace
@@ -549,10 +655,9 @@ int launch_chain(cpipe_cuda_chain* c, const void* d_raw, size_t raw_pitch, void*
     const Img mid1{c->d_mid[1], w, h, (long long)w * 4, 4};
     const int out_elem = c->display == 1 ? 1 : (c->display == 2 ? 2 : elem);
     const Img out{d_out, w, h, (long long)(out_pitch ? out_pitch / out_elem : (size_t)w * 4), 4};
-    const dim3 ga((unsigned)((w + kDmTW - 1) / kDmTW), (unsigned)((h + kDmTH - 1) / kDmTH));
-#define K1(A)                                                                                        \
-    if (c->f16) raw_to_rgba_kernel<A, __half><<<ga, 256, 0, st>>>(raw, mid0, c->raw);                \
-    else raw_to_rgba_kernel<A, float><<<ga, 256, 0, st>>>(raw, mid0, c->raw);
+#define K1(A)                                                          \
+    if (c->f16) launch_raw_to_rgba<A, __half>(raw, mid0, c->raw, st);  \
+    else launch_raw_to_rgba<A, float>(raw, mid0, c->raw, st);
     if (c->algo == 0) { K1(0) } else if (c->algo == 1) { K1(1) } else { K1(2) }
 #undef K1
     if (ev) cudaEventRecord(ev[1], st);
@@ -628,9 +733,7 @@ int launch_chain(cpipe_cuda_chain* c, const void* d_raw, size_t raw_pitch, void*
     // with finishing stages the tone kernel writes a scratch frame they read
     const bool finish = c->sharpen || c->display != 0;
     const Img k3_out = !finish ? out : (k2_out.data == mid0.data ? mid1 : mid0);
-    const dim3 gc((unsigned)((w + kCTW - 1) / kCTW), (unsigned)((h + kCTH - 1) / kCTH));
-#define K3(TT, F, R)                                                                                       \
-    denoise_tone_kernel<TT, F, R><<<gc, 256, denoise_tone_smem<TT, F, R>(), st>>>(k2_out, k3_out, c->tone);
+#define K3(TT, F, R) launch_tone<TT, F, R>(k2_out, k3_out, c->tone, st);
     if (c->f16) {
         if (c->radius == 0) { K3(__half, true, 0) } else if (c->radius == 1) { K3(__half, true, 1) } else { K3(__half, true, 2) }
     } else {
@@ -655,12 +758,11 @@ int launch_chain(cpipe_cuda_chain* c, const void* d_raw, size_t raw_pitch, void*
 
 template <class T, bool F, int R>
 cudaError_t allow_smem() {
-    cudaError_t e = cudaFuncSetAttribute(denoise_tone_kernel<T, F, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)denoise_tone_smem<T, F, R>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(denoise_tone_kernel<T, F, R>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
-    return e;
+    auto* k = denoise_tone_kernel<T, F, R, kCTW, kCTH>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ToneGeom<R, kCTW, kCTH>::bytes());
+    if (e == cudaSuccess && R > 0)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;  // (the small tile stays within the default)
 }
 
 }  // namespace
@@ -1286,7 +1388,7 @@ __global__ void __launch_bounds__(128) batch_color_kernel(const Frame* __restric
 }
 
 template <int R>
-__global__ void __launch_bounds__(256, 3) batch_tone_kernel(const Frame* __restrict__ frames,
+__global__ void __launch_bounds__(256, 4) batch_tone_kernel(const Frame* __restrict__ frames,
                                                             const int* __restrict__ prefix, int n,
                                                             int* __restrict__ left,
                                                             unsigned long long* __restrict__ done) {
@@ -1354,11 +1456,11 @@ int batch_launch_stage(cpipe_cuda_batch* b, int stage, cudaStream_t st, bool tim
         int* left = timed ? b->d_left : nullptr;
         unsigned long long* done = b->d_times + 1;
         if (b->radius == 0)
-            cpb::batch::batch_tone_kernel<0><<<grid, 256, denoise_tone_smem<__half, true, 0>(), st>>>(b->d_frames, pf, b->n, left, done);
+            cpb::batch::batch_tone_kernel<0><<<grid, 256, ToneGeom<0, kCTW, kCTH>::bytes(), st>>>(b->d_frames, pf, b->n, left, done);
         else if (b->radius == 1)
-            cpb::batch::batch_tone_kernel<1><<<grid, 256, denoise_tone_smem<__half, true, 1>(), st>>>(b->d_frames, pf, b->n, left, done);
+            cpb::batch::batch_tone_kernel<1><<<grid, 256, ToneGeom<1, kCTW, kCTH>::bytes(), st>>>(b->d_frames, pf, b->n, left, done);
         else
-            cpb::batch::batch_tone_kernel<2><<<grid, 256, denoise_tone_smem<__half, true, 2>(), st>>>(b->d_frames, pf, b->n, left, done);
+            cpb::batch::batch_tone_kernel<2><<<grid, 256, ToneGeom<2, kCTW, kCTH>::bytes(), st>>>(b->d_frames, pf, b->n, left, done);
     }
     return cuda_status(cudaGetLastError(), "batch stage");
 }
@@ -1408,7 +1510,7 @@ int batch_prefix(cpipe_cuda_batch* b) {
 template <int R>
 cudaError_t allow_batch_smem() {
     cudaError_t e = cudaFuncSetAttribute(cpb::batch::batch_tone_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)denoise_tone_smem<__half, true, R>());
+                                         (int)ToneGeom<R, kCTW, kCTH>::bytes());
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(cpb::batch::batch_tone_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);

@@ -9,8 +9,9 @@
 namespace cpb {
 
 constexpr int kDmTW = 64, kDmTH = 16, kDmHalo = 3, kDmThreads = 256;
-constexpr int kDmIW = kDmTW + 2 * kDmHalo, kDmIH = kDmTH + 2 * kDmHalo;
-constexpr int kDmGW = kDmTW + 2, kDmGH = kDmTH + 2;
+// Quarter-size tiles, for frames of fewer full tiles than SMs (bound by one
+// tile's latency: 160 x 120 through the chain's first kernel, 8.2 us with full tiles).
+constexpr int kDmTWs = 32, kDmTHs = 8;
 
 struct DmTap {
     const float* base;
@@ -20,25 +21,26 @@ struct DmTap {
 
 // Staged halo: RCD / AMaZE read green / chroma at +-1 whose stencils reach
 // +-2 (halo 3); bilinear reads +-1 only (halo 1, a smaller tile to load).
-template <int ALGO>
+template <int ALGO, int TW, int TH>
 struct DmGeom {
     static constexpr int kHalo = ALGO == 0 ? 1 : kDmHalo;
-    static constexpr int kIW = kDmTW + 2 * kHalo, kIH = kDmTH + 2 * kHalo;
+    static constexpr int kIW = TW + 2 * kHalo, kIH = TH + 2 * kHalo;
 };
 
-// Tile of kDmTW x kDmTH outputs; shared memory holds the loaded input with a
+// Tile of TW x TH outputs; shared memory holds the loaded input with a
 // halo of 3 (RCD/AMaZE read green/chroma at +-1 whose stencils reach +-2), and
 // for the tile plus a halo of 1 the green plane and the per-cell quantity the
 // neighbours read: the RCD ratio c / max(g, 1e-6) (demosaic_rcd_generator.cpp:37-40)
 // or the AMaZE chroma c - g (demosaic_amaze_generator.cpp:48-49), computed once
 // per cell instead of once per reading pixel (same values).
-template <int ALGO, class TOut, class Loader>
+template <int ALGO, class TOut, int TW = kDmTW, int TH = kDmTH, class Loader>
 __device__ __forceinline__ void demosaic_tile_at(const Loader& load, int w, int h, const Img& out, const Cfa& cfa, int x0,
                                                  int y0) {
-    constexpr int HL = DmGeom<ALGO>::kHalo, IW = DmGeom<ALGO>::kIW, IH = DmGeom<ALGO>::kIH;
+    using Gm = DmGeom<ALGO, TW, TH>;
+    constexpr int HL = Gm::kHalo, IW = Gm::kIW, IH = Gm::kIH, GW = TW + 2, GH = TH + 2;
     __shared__ float s_in[IH * IW];
-    __shared__ float s_g[ALGO != 0 ? kDmGH * kDmGW : 1];
-    __shared__ float s_q[ALGO != 0 ? kDmGH * kDmGW : 1];
+    __shared__ float s_g[ALGO != 0 ? GH * GW : 1];
+    __shared__ float s_q[ALGO != 0 ? GH * GW : 1];
     // Every caller launches kDmThreads threads per block; a thread's tile loads
     // are all issued before its first shared-memory store.
     constexpr int kLoads = (IH * IW + kDmThreads - 1) / kDmThreads;
@@ -56,8 +58,8 @@ __device__ __forceinline__ void demosaic_tile_at(const Loader& load, int w, int 
     }
     __syncthreads();
     if (ALGO != 0) {
-        for (int i = threadIdx.x; i < kDmGH * kDmGW; i += blockDim.x) {
-            const int ty = i / kDmGW, tx = i - ty * kDmGW;
+        for (int i = threadIdx.x; i < GH * GW; i += blockDim.x) {
+            const int ty = i / GW, tx = i - ty * GW;
             const DmTap T{s_in + (ty + HL - 1) * IW + (tx + HL - 1), IW};
             const float g = ALGO == 1 ? rcd_green(T, x0 - 1 + tx, y0 - 1 + ty, cfa)
                                       : amaze_green(T, x0 - 1 + tx, y0 - 1 + ty, cfa);
@@ -66,8 +68,8 @@ __device__ __forceinline__ void demosaic_tile_at(const Loader& load, int w, int 
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < kDmTH * kDmTW; i += blockDim.x) {
-        const int ty = i / kDmTW, tx = i - ty * kDmTW;
+    for (int i = threadIdx.x; i < TH * TW; i += blockDim.x) {
+        const int ty = i / TW, tx = i - ty * TW;
         const int x = x0 + tx, y = y0 + ty;
         if (x >= out.w || y >= out.h) continue;
         const float* c = s_in + (ty + HL) * IW + (tx + HL);
@@ -86,9 +88,9 @@ __device__ __forceinline__ void demosaic_tile_at(const Loader& load, int w, int 
             g = (red || blue) ? cross : ctr;
             b = blue ? ctr : red ? diag : hred ? vt : hz;
         } else {
-            const float gc = s_g[(ty + 1) * kDmGW + (tx + 1)];
-            const float* Q = s_q + (ty + 1) * kDmGW + (tx + 1);
-#define QQ(dx, dy) Q[(dy) * kDmGW + (dx)]
+            const float gc = s_g[(ty + 1) * GW + (tx + 1)];
+            const float* Q = s_q + (ty + 1) * GW + (tx + 1);
+#define QQ(dx, dy) Q[(dy) * GW + (dx)]
             if (ALGO == 1) {  // demosaic_rcd_generator.cpp:41-63
                 const float rh = gc * 0.5F * (QQ(-1, 0) + QQ(1, 0));
                 const float rv = gc * 0.5F * (QQ(0, -1) + QQ(0, 1));
@@ -111,10 +113,10 @@ __device__ __forceinline__ void demosaic_tile_at(const Loader& load, int w, int 
     }
 }
 
-// One kDmTW x kDmTH tile at the block's grid position.
-template <int ALGO, class TOut, class Loader>
+// One TW x TH tile at the block's grid position.
+template <int ALGO, class TOut, int TW = kDmTW, int TH = kDmTH, class Loader>
 __device__ __forceinline__ void demosaic_tile(const Loader& load, int w, int h, const Img& out, const Cfa& cfa) {
-    demosaic_tile_at<ALGO, TOut>(load, w, h, out, cfa, (int)blockIdx.x * kDmTW, (int)blockIdx.y * kDmTH);
+    demosaic_tile_at<ALGO, TOut, TW, TH>(load, w, h, out, cfa, (int)blockIdx.x * TW, (int)blockIdx.y * TH);
 }
 
 }  // namespace cpb

@@ -138,6 +138,15 @@ __device__ __forceinline__ float const_div(float x, const ConstDiv& c) {
     return __fmaf_rn(r, c.inv, q0);
 }
 
+// Both components by const_div's method, two to an instruction (a fused
+// multiply-add per step, so nothing is contracted that was not).
+static __device__ __noinline__ float2 const_div2_any(float2 v, float d) { return make_float2(v.x / d, v.y / d); }
+__device__ __forceinline__ float2 const_div2(const float2& v, const ConstDiv& c) {
+    if (!(const_div_ok(v.x) && const_div_ok(v.y))) return const_div2_any(v, c.d);
+    const float2 inv = make_float2(c.inv, c.inv), q0 = make_float2(__fmul_rn(v.x, c.inv), __fmul_rn(v.y, c.inv));
+    return __ffma2_rn(__ffma2_rn(q0, make_float2(-c.d, -c.d), v), inv, q0);
+}
+
 // filmic_rgb_generator.cpp:22-36,57-70.  exposure = pow(2, ev) and
 // inv_contrast = 1/contrast are computed once per launch on the host with the
 // same float operations; log_white = log(109) is the generator's constant.
@@ -303,6 +312,19 @@ __device__ __forceinline__ Rgba wavelet_px(const Rgba q[4], const Rgba& p, int o
     const float co = haar_pick(bco, ox, oy), cg = haar_pick(bcg, ox, oy);
     const float t = luma - (0.5F * cg);
     return Rgba{max0(t + (0.5F * co)), max0(t + cg), max0(t - (0.5F * co)), max0(p.a)};
+}
+
+// All four pixels of an aligned block at once (in place): wavelet_px's results, the bands computed once.
+__device__ __forceinline__ void wavelet_block(Rgba (&q)[4], float th) {
+    const HaarBand bco = haar_shrink(wv_co(q[0]), wv_co(q[1]), wv_co(q[2]), wv_co(q[3]), th);
+    const HaarBand bcg = haar_shrink(wv_cg(q[0]), wv_cg(q[1]), wv_cg(q[2]), wv_cg(q[3]), th);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float luma = (q[k].r + (2.0F * q[k].g) + q[k].b) * 0.25F;
+        const float co = haar_pick(bco, k & 1, k >> 1), cg = haar_pick(bcg, k & 1, k >> 1);
+        const float t = luma - (0.5F * cg);
+        q[k] = Rgba{max0(t + (0.5F * co)), max0(t + cg), max0(t - (0.5F * co)), max0(q[k].a)};
+    }
 }
 
 // --------------------------------------------------------------- OpcodeList3

@@ -142,6 +142,19 @@ def test_chain_equals_nodes_on_gpu(cuda_device, host):
     chain.close()
 
 
+# 147 and 150 tiles of 64 x 16 (the quarter-size tiles end below one tile per SM), ragged edges on both sides of the
+# line, odd frames whose last 2x2 blocks are cut, frames narrower than a block column; guided radius 0, 1 and 2
+@pytest.mark.parametrize("radius", [0, 1, 8])
+@pytest.mark.parametrize("w,h", [(448, 336), (640, 240), (575, 257), (577, 255), (33, 9), (31, 7), (1, 3), (2, 1)])
+def test_chain_tile_sizes_equal_nodes(cuda_device, host, w, h, radius):
+    cfg = ChainConfig.small(w, h, guided_radius=radius)
+    raw = cfg.make_raw() if min(w, h) > 8 else np.random.default_rng(w).integers(16, 1023, (h, w)).astype(np.uint16)
+    chain = Chain(cfg)
+    fused = chain.run_host(raw)
+    assert f16_ulp_distance(fused, run_nodes_on_gpu(host, cfg, raw)).max() == 0
+    chain.close()
+
+
 def test_chain_general_opcode_list(cuda_device):
     """OpcodeList3 lists other than a single warp take the per-node path inside the chain."""
     import ctypes as C
