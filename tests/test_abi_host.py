@@ -202,3 +202,23 @@ def test_cube_loader(tmp_path):
     out = np.zeros(24, np.float32)
     assert L.cpipe_b200_load_lut(spi.encode(), C.byref(size), out.ctypes.data, out.size) == _abi.OK
     assert size.value == 2 and out[-3:].tolist() == [0.5, 0.25, 0.75]
+
+
+@pytest.mark.parametrize("form", ["{:.9g}", "{:.18f}", "{:+.6e}", "{:.3f}", "mid"])
+def test_cube_number_forms_round_like_strtof(tmp_path, form):
+    """Plain decimals, exponents, signs, more digits than a double holds and middles between two floats: each row's
+    value is the correctly rounded binary32, whichever way the loader reads the row."""
+    S = 8
+    v = np.random.default_rng(5).uniform(-2, 2, size=S ** 3 * 3).astype(np.float32)
+    mids = (v.astype(np.float64) + np.nextafter(v, np.float32(9)).astype(np.float64)) / 2  # exact in a double
+    text = ["{:.17f}".format(m) if form == "mid" else form.format(float(x)) for x, m in zip(v, mids)]
+    path = str(tmp_path / "n.cube")
+    with open(path, "w", newline="") as f:
+        f.write(f"TITLE x\r\nLUT_3D_SIZE {S}\r\n")
+        f.writelines("\t".join(text[i:i + 3]) + " # row\r\n" for i in range(0, len(text), 3))
+    size, out = C.c_uint32(), np.zeros(v.size, np.float32)
+    assert _abi.lib().cpipe_b200_load_lut(path.encode(), C.byref(size), out.ctypes.data, out.size) == _abi.OK
+    libc = C.CDLL(None)
+    libc.strtof.restype, libc.strtof.argtypes = C.c_float, [C.c_char_p, C.c_void_p]
+    want = np.array([libc.strtof(t.encode(), None) for t in text], np.float32)
+    np.testing.assert_array_equal(out.view(np.uint32), want.view(np.uint32))
