@@ -93,15 +93,17 @@ __device__ __forceinline__ bool gated_off(const int* gate) { return gate != null
 template <class T>
 __global__ void bm3d_prep_kernel(Img in, float* __restrict__ yuv, uint8_t* __restrict__ q, long long npx,
                                  const int* gate) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= in.w || gated_off(gate)) return;
-    const Rgba p = load_rgba(px<const T>(in, x, y));
-    const float s = (p.r + p.g) + p.b;
-    const long long o = (long long)y * in.w + x;
-    yuv[o] = s * kInvS3;
-    yuv[npx + o] = (p.r - p.b) * kInvS2;
-    yuv[2 * npx + o] = ((p.r + p.b) - 2.0F * p.g) * kInvS6;
-    q[o] = quantise(s * (1.0F / 3.0F));
+    for (int y = blockIdx.y; y < in.h; y += gridDim.y) {
+        const Rgba p = load_rgba(px<const T>(in, x, y));
+        const float s = (p.r + p.g) + p.b;
+        const long long o = (long long)y * in.w + x;
+        yuv[o] = s * kInvS3;
+        yuv[npx + o] = (p.r - p.b) * kInvS2;
+        yuv[2 * npx + o] = ((p.r + p.b) - 2.0F * p.g) * kInvS6;
+        q[o] = quantise(s * (1.0F / 3.0F));
+    }
 }
 
 // ------------------------------------------------------------------ match
@@ -883,12 +885,10 @@ __host__ __device__ constexpr int tc_stage_blocks(int stage) { return stage == 2
 //                atomic per block), and the separable Kaiser window is applied
 //                to that map at the flush.
 template <int STAGE, bool SPLIT>
-__global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_kernel(FilterArgs a) {
+__device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int ty, int c, int img) {
     constexpr int SB = tc_stage_blocks(STAGE);
     extern __shared__ __align__(16) float sm[];
-    const int c = blockIdx.z % 3, img = blockIdx.z / 3, row0 = img * a.h;
-    const int tx = blockIdx.x, ty = blockIdx.y;
-    if (tx >= a.ntx || ty >= a.nty || gated_off(a.gate)) return;
+    const int row0 = img * a.h;
     const int i0 = tx * kRefTile, j0 = ty * kRefTile;
     const int i1 = min(i0 + kRefTile, a.nrx), j1 = min(j0 + kRefTile, a.nry);
     const int fx0 = max(0, refpos(i0, a.w, a.nstep) - a.R);
@@ -1072,32 +1072,53 @@ __global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_kernel(Filter
     }
 }
 
+template <int STAGE, bool SPLIT>
+__global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_kernel(const __grid_constant__ FilterArgs a) {
+    filter_tc_tile<STAGE, SPLIT>(a, blockIdx.x, blockIdx.y, blockIdx.z % 3, blockIdx.z / 3);
+}
+// A gated run seldom happens: a grid of resident CTAs that walk the tiles, so
+// that one which does not costs the launch (3 us) and not the start of every
+// tile's CTA (46 us a stage at 12 MP).
+template <int STAGE, bool SPLIT>
+__global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_gated_kernel(const __grid_constant__ FilterArgs a,
+                                                                               int tiles) {
+    if (gated_off(a.gate)) return;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int z = t / (a.ntx * a.nty), r = t - z * (a.ntx * a.nty);
+        filter_tc_tile<STAGE, SPLIT>(a, r % a.ntx, r / a.ntx, z % 3, z / 3);
+        __syncthreads();
+    }
+}
+
 // --------------------------------------------------------- basic / final
 __global__ void bm3d_basic_kernel(const float* __restrict__ acc, float* __restrict__ basic, uint8_t* __restrict__ q,
                                   long long npx, const int* gate) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npx || gated_off(gate)) return;
-    float y = 0.0F;
+    if (gated_off(gate)) return;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += (long long)gridDim.x * blockDim.x) {
+        float y = 0.0F;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float v = acc[c * npx + i] / acc[(3 + c) * npx + i];
-        basic[c * npx + i] = v;
-        if (c == 0) y = v;
+        for (int c = 0; c < 3; ++c) {
+            const float v = acc[c * npx + i] / acc[(3 + c) * npx + i];
+            basic[c * npx + i] = v;
+            if (c == 0) y = v;
+        }
+        q[i] = quantise(y * kInvS3);
     }
-    q[i] = quantise(y * kInvS3);
 }
 
 template <class T>
 __global__ void bm3d_final_kernel(const float* __restrict__ acc, Img in, Img out, long long npx, const int* gate) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= in.w || gated_off(gate)) return;
-    const long long i = (long long)y * in.w + x;
-    const float Y = acc[i] / acc[3 * npx + i];
-    const float U = acc[npx + i] / acc[4 * npx + i];
-    const float V = acc[2 * npx + i] / acc[5 * npx + i];
-    const float yy = Y * kInvS3, uu = U * kInvS2, vv = V * kInvS6;
-    const Rgba o{(yy + uu) + vv, yy - 2.0F * vv, (yy - uu) + vv, 0.0F};
-    store_rgb_keep_alpha(px<T>(out, x, y), o, px<const T>(in, x, y));
+    for (int y = blockIdx.y; y < in.h; y += gridDim.y) {
+        const long long i = (long long)y * in.w + x;
+        const float Y = acc[i] / acc[3 * npx + i];
+        const float U = acc[npx + i] / acc[4 * npx + i];
+        const float V = acc[2 * npx + i] / acc[5 * npx + i];
+        const float yy = Y * kInvS3, uu = U * kInvS2, vv = V * kInvS6;
+        const Rgba o{(yy + uu) + vv, yy - 2.0F * vv, (yy - uu) + vv, 0.0F};
+        store_rgb_keep_alpha(px<T>(out, x, y), o, px<const T>(in, x, y));
+    }
 }
 
 __global__ void bm3d_zero_kernel(float* __restrict__ p, long long n, const int* gate) {
@@ -1240,6 +1261,10 @@ cudaError_t bm3d_setup(const Bm3dPlan& p) {
         if (t2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
         const void* k1 = p.split ? (const void*)bm3d_filter_tc_kernel<1, true> : (const void*)bm3d_filter_tc_kernel<1, false>;
         const void* k2 = p.split ? (const void*)bm3d_filter_tc_kernel<2, true> : (const void*)bm3d_filter_tc_kernel<2, false>;
+        const void* g1 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<1, true> : (const void*)bm3d_filter_tc_gated_kernel<1, false>;
+        const void* g2 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<2, true> : (const void*)bm3d_filter_tc_gated_kernel<2, false>;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t2);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t1);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t2);
     }
@@ -1267,7 +1292,11 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     const size_t fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
     const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
 
-    const dim3 pgrid((p.w + 255) / 256, p.h * p.batch);
+    // a gated run's kernels walk the frame with few CTAs: it seldom happens, and
+    // should not cost the start of a CTA for every row when it does not
+    const int prows = gate ? std::min(p.h * p.batch, std::max(1, 8 * kSmCount / ((p.w + 255) / 256))) : p.h * p.batch;
+    const dim3 pgrid((p.w + 255) / 256, prows);
+    const unsigned bgrid = (unsigned)(gate ? std::min((npx + 255) / 256, (long long)kSmCount * 8) : (npx + 255) / 256);
     if (f16) bm3d_prep_kernel<__half><<<pgrid, 256, 0, st>>>(in, yuv, q, npx, gate);
     else bm3d_prep_kernel<float><<<pgrid, 256, 0, st>>>(in, yuv, q, npx, gate);
 
@@ -1306,7 +1335,16 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
         bm3d_zero_kernel<<<kSmCount * 8, 256, 0, st>>>(acc, 6 * npx, gate);
         ma.dthr = p.dthr[stage - 1];
         bm3d_match_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
-        if (p.tensor) {
+        if (p.tensor && gate) {
+            const int tiles = p.ntx * p.nty * 3 * p.batch, g = std::min(tiles, kSmCount * 3);
+            if (p.split) {
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, true><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, true><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
+            } else {
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, false><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, false><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
+            }
+        } else if (p.tensor) {
             if (p.split) {
                 if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);
                 else bm3d_filter_tc_kernel<2, true><<<tgrid, 32 * kTcWarps, ts2, st>>>(ta);
@@ -1322,7 +1360,7 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
                 }
         }
         if (stage == 1 && p.stages == 2)
-            bm3d_basic_kernel<<<(unsigned)((npx + 255) / 256), 256, 0, st>>>(acc, basic, q, npx, gate);
+            bm3d_basic_kernel<<<bgrid, 256, 0, st>>>(acc, basic, q, npx, gate);
     }
     if (f16) bm3d_final_kernel<__half><<<pgrid, 256, 0, st>>>(acc, in, out, npx, gate);
     else bm3d_final_kernel<float><<<pgrid, 256, 0, st>>>(acc, in, out, npx, gate);

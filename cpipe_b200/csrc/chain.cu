@@ -494,11 +494,14 @@ __global__ void decide_kernel(const float* __restrict__ part, int n, int edge, f
                               SpotStats* stats) {
     const int chunks = (edge + kMseRows - 1) / kMseRows;
     float worst = 0.0F;
-    for (int t = 0; t < n; ++t) {
+    if ((int)threadIdx.x < n) {  // a lane per tile (one thread for all of them took 13 us)
         float s = 0.0F;
-        for (int k = 0; k < chunks; ++k) s += part[t * kMseChunks + k];
+        for (int k = 0; k < chunks; ++k) s += part[threadIdx.x * kMseChunks + k];
         worst = fmaxf(worst, s / (3.0F * (float)(edge * edge)));
     }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xFFFFFFFFU, worst, off));
+    if (threadIdx.x != 0) return;
     const int fall = !(worst <= mse_max);  // a non-finite tile error also falls back
     *gate = fall;
     stats->frames += 1U;
@@ -632,7 +635,7 @@ int denoise_stage(cpipe_cuda_chain* c, const Img& k2_out, const Img& dn_out, cud
         const dim3 gm((unsigned)((E + spot::kMseRows - 1) / spot::kMseRows), (unsigned)n);
         if (c->f16) spot::mse_kernel<__half><<<gm, 256, 0, st>>>(dn_out, static_cast<const __half*>(c->d_tile_ref), E, c->spot, c->d_tile_mse);
         else spot::mse_kernel<float><<<gm, 256, 0, st>>>(dn_out, static_cast<const float*>(c->d_tile_ref), E, c->spot, c->d_tile_mse);
-        spot::decide_kernel<<<1, 1, 0, st>>>(c->d_tile_mse, n, E, c->spot_mse_max, c->d_gate, c->d_stats);
+        spot::decide_kernel<<<1, 32, 0, st>>>(c->d_tile_mse, n, E, c->spot_mse_max, c->d_gate, c->d_stats);
         e = bm3d_run(c->bm3d, k2_out, dn_out, c->f16, c->d_denoise, st, false, c->d_gate);
     }
     return e == cudaSuccess ? CPIPE_OK : cuda_status(e, "chain denoise");
