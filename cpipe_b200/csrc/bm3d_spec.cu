@@ -817,18 +817,16 @@ template <bool SPLIT>
 __device__ __forceinline__ void tc_forward(const float* img, int P, const int* off, int N, const DctFrags& d,
                                            float (&H)[8][4]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    img += 2 * q * P + g;
+    int4 o = make_int4(0, 0, 0, 0);
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
         H[t][0] = H[t][1] = H[t][2] = H[t][3] = 0.0F;
         if (2 * t >= N) continue;
-        float v[2][2] = {{0.0F, 0.0F}, {0.0F, 0.0F}};
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh)
-            if (2 * t + hh < N) {
-                const float* src = img + off[2 * t + hh] + 2 * q * P + g;
-                v[hh][0] = src[0];
-                v[hh][1] = src[P];
-            }
+        if (t % 2 == 0) o = *reinterpret_cast<const int4*>(off + 2 * t);
+        const int o0 = t % 2 ? o.z : o.x, o1 = t % 2 ? o.w : o.y;
+        float v[2][2] = {{img[o0], img[o0 + P]}, {0.0F, 0.0F}};
+        if (2 * t + 1 < N) v[1][0] = img[o1], v[1][1] = img[o1 + P];
         float rc[4];
         mma_prod<SPLIT>(rc, v[0][0], v[0][1], v[1][0], v[1][1], d.fh, d.fl);  // rows (block, x = g), columns v
         mma_prod_t<SPLIT>(H[t], rc, d.fh, d.fl);                             // rows (block, v = g), columns u
@@ -867,26 +865,28 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 constexpr int kTcWarps = 8;
-constexpr int kStageStride = 72;  // floats per block in a warp's staging buffer (64 + 8: conflict-free float2 stores)
-// blocks staged per round: 4 in stage 2 keeps three CTAs of it within one SM's shared memory
-__host__ __device__ constexpr int tc_stage_blocks(int stage) { return stage == 2 ? 4 : 8; }
 
 // One launch per stage covers every tile: footprints of neighbouring tiles
 // overlap, and the flush adds into the frame accumulators with global
 // reductions.  The footprint planes use a row pitch P = 4 mod 32 (>= the
 // footprint edge), which makes the column loads of the forward transform and
 // the numerator atomics fall in 32 different banks.  Aggregation inside a tile:
-//   numerator    the group's inverse-transformed blocks go through the warp's
-//                staging buffer ([block][x][y]), so each shared-memory atomic
-//                instruction covers 32 distinct pixels (8 rows x 4 columns) of
-//                one block;
+//   numerator    added from the inverse transform's accumulators: a lane holds
+//                two rows of one column, so each shared-memory atomic
+//                instruction covers 32 distinct pixels of one block in 32 banks
+//                (a staging buffer in between cost 48 shared accesses a group
+//                and channel);
 //   denominator  sum over placements of weight x Kaiser(pixel - origin): the
 //                weights are added at the block origins (a weight map, one
 //                atomic per block), and the separable Kaiser window is applied
-//                to that map at the flush.
+//                to that map at the flush, four columns to a thread.
+// Bound by issue (the split products' MMAs and splits, a Haar tree, the
+// atomics), so what is not arithmetic counts: block offsets are read four at a
+// time, nothing is staged.  12 MP chain frame, split products: stage 1 11.3 ->
+// 9.8 ms, stage 2 15.5 -> 13.0 ms against a form with a staging buffer, an
+// offset load per block and a scalar flush.
 template <int STAGE, bool SPLIT>
 __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int ty, int c, int img) {
-    constexpr int SB = tc_stage_blocks(STAGE);
     extern __shared__ __align__(16) float sm[];
     const int row0 = img * a.h;
     const int i0 = tx * kRefTile, j0 = ty * kRefTile;
@@ -900,11 +900,9 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* s_num = sm;
     float* s_img = sm + FP;                             // after the groups: the weight map, then den
-    float* s_bas = s_img + FP;                          // stage 2
-    float* s_aux = s_img + (STAGE == 2 ? 2 : 1) * FP;  // staging buffers (stage 1: at the flush the row-filtered map)
-    float* s_k = s_aux + (STAGE == 2 ? kTcWarps * SB * kStageStride : max(FP, kTcWarps * SB * kStageStride));
-    float* s_k1 = s_k + 64;
-    float* s_wgt = s_k1 + 8;  // one aggregation weight per reference block of the tile
+    float* s_bas = s_img + FP;                          // stage 2 (s_row at the flush)
+    float* s_row = s_img + FP;  // the footprint of the basic estimate in stage 2; at the flush the row-filtered map
+    float* s_wgt = s_row + FP;  // one aggregation weight per reference block of the tile
     uint32_t* s_list = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_wgt + kRefTile * kRefTile) + 15) &
                                                    ~(uintptr_t)15);
     uint32_t* s_cnt = s_list + kRefTile * kRefTile * 16;
@@ -928,9 +926,8 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         const int k = threadIdx.x;
         s_cnt[k] = a.cnt[((long long)img * a.nry + j0 + k / nti) * a.nrx + i0 + k % nti];
     }
-    for (int idx = threadIdx.x; idx < FP; idx += blockDim.x) s_num[idx] = 0.0F;
-    if (threadIdx.x < 64) s_k[threadIdx.x] = a.kaiser[threadIdx.x];
-    if (threadIdx.x < 8) s_k1[threadIdx.x] = a.kaiser1[threadIdx.x];
+    const float4 zero4 = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+    for (int idx = threadIdx.x; idx < FP / 4; idx += blockDim.x) reinterpret_cast<float4*>(s_num)[idx] = zero4;
     cp_async_wait_all();
     __syncthreads();
 
@@ -939,9 +936,8 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
     // hard thresholds of the unnormalised coefficients: lambda sigma 2^(k/2)
     const float thr1 = a.thr * 1.41421356237309515F, thr2 = a.thr * 2.0F, thr3 = a.thr * 2.82842712474619030F,
                 thr4 = a.thr * 4.0F;
-    float* stg = s_aux + warp * (SB * kStageStride);
-    const int ly = lane & 7, lx = lane >> 3;  // a lane's pixel in an 8x4 half-block (y, x) and (y, x + 4)
-    const float kq0 = s_k[ly * 8 + lx], kq1 = s_k[ly * 8 + lx + 4];
+    // the window at the lane's two pixels of a block, (x, y) = (g, 2q) and (g, 2q + 1)
+    const float kq0 = a.kaiser[2 * q * 8 + g], kq1 = a.kaiser[(2 * q + 1) * 8 + g];
     for (int k = warp; k < nref; k += kTcWarps) {
         const int cnt = (int)s_cnt[k];
         const int N = cnt >= 16 ? 16 : cnt >= 8 ? 8 : cnt >= 4 ? 4 : cnt >= 2 ? 2 : 1;
@@ -998,33 +994,29 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         if (lane == 0) s_wgt[k] = wgt;
         float X[8][4];
         tc_inverse<SPLIT>(H, N, dct, X);
-        // numerator: X -> staging [block][x][y], SB blocks per round -> one block's
-        // 8x4 half per atomic instruction
+        // numerator, straight from the accumulators: an atomic instruction covers
+        // 8 columns x every other row of a block, 32 pixels in 32 banks (P = 4 mod 32)
         const float kw0 = wgt * kq0, kw1 = wgt * kq1;
+        float* num = s_num + 2 * q * P + g;
+        int4 o = make_int4(0, 0, 0, 0);
 #pragma unroll
-        for (int rb = 0; rb < 16 / SB; ++rb) {
-            if (SB * rb >= N) break;
-#pragma unroll
-            for (int tt = 0; tt < SB / 2; ++tt) {
-                const int t = rb * (SB / 2) + tt;
-                *reinterpret_cast<float2*>(stg + (2 * tt) * kStageStride + g * 8 + 2 * q) = make_float2(X[t][0], X[t][1]);
-                *reinterpret_cast<float2*>(stg + (2 * tt + 1) * kStageStride + g * 8 + 2 * q) =
-                    make_float2(X[t][2], X[t][3]);
+        for (int t = 0; t < 8; ++t) {
+            if (2 * t >= N) break;
+            if (t % 2 == 0) o = *reinterpret_cast<const int4*>(woff + 2 * t);
+            float* d0 = num + (t % 2 ? o.z : o.x);
+            atomicAdd(d0, kw0 * X[t][0]);
+            atomicAdd(d0 + P, kw1 * X[t][1]);
+            if (2 * t + 1 < N) {
+                float* d1 = num + (t % 2 ? o.w : o.y);
+                atomicAdd(d1, kw0 * X[t][2]);
+                atomicAdd(d1 + P, kw1 * X[t][3]);
             }
-            __syncwarp();
-            const int nb = min(SB, N - SB * rb);
-            for (int bb = 0; bb < nb; ++bb) {
-                float* dst = s_num + woff[SB * rb + bb] + ly * P + lx;
-                atomicAdd(dst, kw0 * stg[bb * kStageStride + lane]);
-                atomicAdd(dst + 4, kw1 * stg[bb * kStageStride + 32 + lane]);
-            }
-            __syncwarp();
         }
     }
     __syncthreads();
     // weight map at the block origins (in the footprint's own plane, now free)
     float* s_w = s_img;
-    for (int idx = threadIdx.x; idx < FP; idx += blockDim.x) s_w[idx] = 0.0F;
+    for (int idx = threadIdx.x; idx < FP / 4; idx += blockDim.x) reinterpret_cast<float4*>(s_w)[idx] = zero4;
     __syncthreads();
     for (int i = threadIdx.x; i < nref * 16; i += blockDim.x) {
         const int k = i >> 4, cnt = (int)s_cnt[k];
@@ -1035,39 +1027,55 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         }
     }
     __syncthreads();
-    // den = map correlated with the Kaiser window: rows into a free plane, then columns
-    float* s_row = STAGE == 2 ? s_bas : s_aux;
-    // (the window comes from the kernel arguments; bounds tests only in the first 7 columns / rows)
-    for (int yy = warp; yy < fh; yy += kTcWarps)
-        for (int xx = lane; xx < fw; xx += 32) {
-            const float* wr = s_w + yy * P + xx;
-            float h = 0.0F;
-            if (xx >= 7) {
+    // den = map correlated with the Kaiser window (from the kernel arguments): rows
+    // into a free plane, then columns, four columns to a thread (16-byte loads);
+    // down the columns a thread keeps the last eight rows in registers
+    const int gx = (fw + 3) / 4;
+    for (int i = threadIdx.x; i < fh * gx; i += blockDim.x) {
+        const int yy = i / gx, xx = 4 * (i - yy * gx);
+        const float4* wr = reinterpret_cast<const float4*>(s_w + yy * P + xx);
+        const float4 w0 = xx >= 8 ? wr[-2] : zero4, w1 = xx >= 4 ? wr[-1] : zero4, w2 = wr[0];
+        const float w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
+        float h[4] = {0.0F, 0.0F, 0.0F, 0.0F};
 #pragma unroll
-                for (int u = 0; u < 8; ++u) h = __fmaf_rn(a.kaiser1[u], wr[-u], h);
-            } else {
-                for (int u = 0; u <= xx; ++u) h = __fmaf_rn(a.kaiser1[u], wr[-u], h);
-            }
-            s_row[yy * P + xx] = h;
-        }
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) h[k] = __fmaf_rn(a.kaiser1[u], w[8 + k - u], h[k]);
+        *reinterpret_cast<float4*>(s_row + yy * P + xx) = make_float4(h[0], h[1], h[2], h[3]);
+    }
     __syncthreads();
     float* gn = a.acc + (long long)c * a.npx;
     float* gd = a.acc + (long long)(3 + c) * a.npx;
-    for (int yy = warp; yy < fh; yy += kTcWarps) {
-        const long long o = (long long)(fy0 + yy) * a.w + fx0;
-        for (int xx = lane; xx < fw; xx += 32) {
-            const float* cr = s_row + yy * P + xx;
-            float d = 0.0F;
-            if (yy >= 7) {
+    const int segs = blockDim.x / gx, seg_rows = (fh + segs - 1) / segs;
+    for (int i = threadIdx.x; i < segs * gx; i += blockDim.x) {
+        const int seg = i / gx, xx = 4 * (i - seg * gx);
+        const int y0 = seg * seg_rows, y1 = min(fh, y0 + seg_rows);
+        if (y0 >= fh) continue;  // (more segments than rows)
+        float4 r[8];             // r[v]: the row v above
 #pragma unroll
-                for (int v = 0; v < 8; ++v) d = __fmaf_rn(a.kaiser1[v], cr[-v * P], d);
-            } else {
-                for (int v = 0; v <= yy; ++v) d = __fmaf_rn(a.kaiser1[v], cr[-v * P], d);
+        for (int v = 1; v < 8; ++v)
+            r[v] = y0 - v >= 0 ? *reinterpret_cast<const float4*>(s_row + (y0 - v) * P + xx) : zero4;
+        for (int yy = y0; yy < y1; ++yy) {
+            r[0] = *reinterpret_cast<const float4*>(s_row + yy * P + xx);
+            float4 d = zero4;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                d.x = __fmaf_rn(a.kaiser1[v], r[v].x, d.x);
+                d.y = __fmaf_rn(a.kaiser1[v], r[v].y, d.y);
+                d.z = __fmaf_rn(a.kaiser1[v], r[v].z, d.z);
+                d.w = __fmaf_rn(a.kaiser1[v], r[v].w, d.w);
             }
-            if (d > 0.0F) {
-                atomicAdd(gn + o + xx, s_num[yy * P + xx]);
-                atomicAdd(gd + o + xx, d);
-            }
+#pragma unroll
+            for (int v = 7; v > 0; --v) r[v] = r[v - 1];
+            const float4 n = *reinterpret_cast<const float4*>(s_num + yy * P + xx);
+            const long long o = (long long)(fy0 + yy) * a.w + fx0 + xx;
+            const float nv[4] = {n.x, n.y, n.z, n.w}, dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (xx + k < fw && dv[k] > 0.0F) {
+                    atomicAdd(gn + o + k, nv[k]);
+                    atomicAdd(gd + o + k, dv[k]);
+                }
         }
     }
 }
@@ -1168,11 +1176,9 @@ size_t match_layout(Bm3dPlan& p, int tile) {
 // 32 (column loads of eight columns x two rows, and atomics of eight rows x
 // four columns, fall in 32 different banks).
 int tile_pitch(int fw) { return fw + ((4 - fw) % 32 + 32) % 32; }
-size_t filter_tc_smem(const Bm3dPlan& p, int stage) {
+size_t filter_tc_smem(const Bm3dPlan& p) {
     const size_t fp = (size_t)p.fw * tile_pitch(p.fw);
-    const size_t stg = (size_t)kTcWarps * tc_stage_blocks(stage) * kStageStride;
-    const size_t aux = stage == 2 ? stg : std::max(fp, stg);
-    const size_t floats = fp + (stage == 2 ? 2 : 1) * fp + aux + 64 + 8 + kRefTile * kRefTile;  // + Kaiser, its 1D factor, weights
+    const size_t floats = 3 * fp + kRefTile * kRefTile;  // numerator, two footprints, weights
     return sizeof(float) * floats + 16 + sizeof(uint32_t) * kRefTile * kRefTile * 17 + sizeof(int) * kTcWarps * 16;
 }
 
@@ -1257,16 +1263,16 @@ cudaError_t bm3d_setup(const Bm3dPlan& p) {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(bm3d_filter_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs2);
     if (p.tensor) {
-        const size_t t1 = filter_tc_smem(p, 1), t2 = filter_tc_smem(p, 2);
-        if (t2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
+        const size_t ts = filter_tc_smem(p);
+        if (ts > kSmemOptIn) return cudaErrorInvalidConfiguration;
         const void* k1 = p.split ? (const void*)bm3d_filter_tc_kernel<1, true> : (const void*)bm3d_filter_tc_kernel<1, false>;
         const void* k2 = p.split ? (const void*)bm3d_filter_tc_kernel<2, true> : (const void*)bm3d_filter_tc_kernel<2, false>;
         const void* g1 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<1, true> : (const void*)bm3d_filter_tc_gated_kernel<1, false>;
         const void* g2 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<2, true> : (const void*)bm3d_filter_tc_gated_kernel<2, false>;
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t2);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t2);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
     }
     return e;
 }
@@ -1290,7 +1296,7 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     cudaError_t e;
     if (setup && (e = bm3d_setup(p)) != cudaSuccess) return e;
     const size_t fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
-    const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
+    const size_t ts = filter_tc_smem(p);
 
     // a gated run's kernels walk the frame with few CTAs: it seldom happens, and
     // should not cost the start of a CTA for every row when it does not
@@ -1338,19 +1344,19 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
         if (p.tensor && gate) {
             const int tiles = p.ntx * p.nty * 3 * p.batch, g = std::min(tiles, kSmCount * 3);
             if (p.split) {
-                if (stage == 1) bm3d_filter_tc_gated_kernel<1, true><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
-                else bm3d_filter_tc_gated_kernel<2, true><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, true><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, true><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
             } else {
-                if (stage == 1) bm3d_filter_tc_gated_kernel<1, false><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
-                else bm3d_filter_tc_gated_kernel<2, false><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, false><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, false><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
             }
         } else if (p.tensor) {
             if (p.split) {
-                if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);
-                else bm3d_filter_tc_kernel<2, true><<<tgrid, 32 * kTcWarps, ts2, st>>>(ta);
+                if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
+                else bm3d_filter_tc_kernel<2, true><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
             } else {
-                if (stage == 1) bm3d_filter_tc_kernel<1, false><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);
-                else bm3d_filter_tc_kernel<2, false><<<tgrid, 32 * kTcWarps, ts2, st>>>(ta);
+                if (stage == 1) bm3d_filter_tc_kernel<1, false><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
+                else bm3d_filter_tc_kernel<2, false><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
             }
         } else {
             for (int py = 0; py < p.phases; ++py)
