@@ -811,47 +811,85 @@ __device__ __forceinline__ constexpr int haar_k(int b) { return (b & 1) ? 1 : (b
 __device__ __forceinline__ float exp2i(int e) { return __int_as_float((127 + e) << 23); }
 
 // Forward 2D DCT and Haar of one group of N blocks read from `img` (row pitch P;
-// off[b]: block b's offset in the footprint plane).  H[t][e]: block 2t (e < 2) or 2t + 1 (e >= 2),
-// coefficient (v = g, u = 2q + (e & 1)).
+// off[b]: block b's offset in the footprint plane, block 0's for b >= N).
+// H[t][e]: block 2t (e < 2) or 2t + 1 (e >= 2), coefficient (v = g, u = 2q + (e & 1)).
+// The pairs of blocks are walked in the segments that a group size of 2, 4, 8 or
+// 16 takes whole, so that a segment's pairs overlap without a branch between them.
 template <bool SPLIT>
 __device__ __forceinline__ void tc_forward(const float* img, int P, const int* off, int N, const DctFrags& d,
                                            float (&H)[8][4]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     img += 2 * q * P + g;
-    int4 o = make_int4(0, 0, 0, 0);
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        H[t][0] = H[t][1] = H[t][2] = H[t][3] = 0.0F;
-        if (2 * t >= N) continue;
-        if (t % 2 == 0) o = *reinterpret_cast<const int4*>(off + 2 * t);
-        const int o0 = t % 2 ? o.z : o.x, o1 = t % 2 ? o.w : o.y;
-        float v[2][2] = {{img[o0], img[o0 + P]}, {0.0F, 0.0F}};
-        if (2 * t + 1 < N) v[1][0] = img[o1], v[1][1] = img[o1 + P];
+    auto pair = [&](int t, int o0, int o1) {
         float rc[4];
-        mma_prod<SPLIT>(rc, v[0][0], v[0][1], v[1][0], v[1][1], d.fh, d.fl);  // rows (block, x = g), columns v
-        mma_prod_t<SPLIT>(H[t], rc, d.fh, d.fl);                             // rows (block, v = g), columns u
-    }
+        mma_prod<SPLIT>(rc, img[o0], img[o0 + P], img[o1], img[o1 + P], d.fh, d.fl);  // rows (block, x = g), columns v
+        mma_prod_t<SPLIT>(H[t], rc, d.fh, d.fl);                                     // rows (block, v = g), columns u
+    };
+    auto segment = [&](int t0, int n) {  // n = 2 or 4 pairs
+#pragma unroll
+        for (int t = t0; t < t0 + n; t += 2) {
+            const int4 o = *reinterpret_cast<const int4*>(off + 2 * t);
+            pair(t, o.x, o.y);
+            pair(t + 1, o.z, o.w);
+        }
+    };
+#pragma unroll
+    for (int t = 0; t < 8; ++t) H[t][0] = H[t][1] = H[t][2] = H[t][3] = 0.0F;
+    const int4 o = *reinterpret_cast<const int4*>(off);
+    pair(0, o.x, o.y);
+    if (N == 1) H[0][2] = H[0][3] = 0.0F;
+    if (N > 2) pair(1, o.z, o.w);
+    if (N > 4) segment(2, 2);
+    if (N > 8) segment(4, 4);
     if (N > 1) haar_level<1>(H);
     if (N > 2) haar_level<2>(H);
     if (N > 4) haar_level<4>(H);
     if (N > 8) haar_level<8>(H);
 }
 
-// Inverse Haar and 2D DCT: X[t][e] = block 2t (e < 2) or 2t + 1, pixel (x = g, y = 2q + (e & 1)).
+// Inverse Haar and 2D DCT of a group; its pixels, weighted by (kw0, kw1), are added
+// to the plane `num` at the blocks' offsets: a lane holds (x = g, y = 2q, 2q + 1) of
+// every block, so an atomic instruction covers 8 columns x every other row of a
+// block, 32 pixels in 32 banks (P = 4 mod 32).
 template <bool SPLIT>
-__device__ __forceinline__ void tc_inverse(float (&H)[8][4], int N, const DctFrags& d, float (&X)[8][4]) {
+__device__ __forceinline__ void tc_inverse_add(float (&H)[8][4], int N, const DctFrags& d, float kw0, float kw1, float* num,
+                                               int P, const int* off) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    num += 2 * q * P + g;
     if (N > 8) haar_level<8>(H);
     if (N > 4) haar_level<4>(H);
     if (N > 2) haar_level<2>(H);
     if (N > 1) haar_level<1>(H);
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        X[t][0] = X[t][1] = X[t][2] = X[t][3] = 0.0F;
-        if (2 * t >= N) continue;
+    auto inverse = [&](int t) {  // in place: pixels (x = g, y = 2q + (e & 1))
         float rr[4];
         mma_prod<SPLIT>(rr, H[t][0], H[t][1], H[t][2], H[t][3], d.ih, d.il);  // rows (block, v = g), columns x
-        mma_prod_t<SPLIT>(X[t], rr, d.ih, d.il);                             // rows (block, x = g), columns y
+        mma_prod_t<SPLIT>(H[t], rr, d.ih, d.il);                             // rows (block, x = g), columns y
+    };
+    auto add = [&](int o, float p0, float p1) {
+        atomicAdd(num + o, kw0 * p0);
+        atomicAdd(num + o + P, kw1 * p1);
+    };
+    auto segment = [&](int t0, int n) {
+#pragma unroll
+        for (int t = t0; t < t0 + n; ++t) inverse(t);
+#pragma unroll
+        for (int t = t0; t < t0 + n; t += 2) {
+            const int4 o = *reinterpret_cast<const int4*>(off + 2 * t);
+            add(o.x, H[t][0], H[t][1]);
+            add(o.y, H[t][2], H[t][3]);
+            add(o.z, H[t + 1][0], H[t + 1][1]);
+            add(o.w, H[t + 1][2], H[t + 1][3]);
+        }
+    };
+    if (N > 2) {
+        segment(0, 2);
+    } else {
+        inverse(0);
+        add(off[0], H[0][0], H[0][1]);
+        if (N > 1) add(off[1], H[0][2], H[0][3]);
     }
+    if (N > 4) segment(2, 2);
+    if (N > 8) segment(4, 4);
 }
 
 __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
@@ -882,9 +920,12 @@ constexpr int kTcWarps = 8;
 //                to that map at the flush, four columns to a thread.
 // Bound by issue (the split products' MMAs and splits, a Haar tree, the
 // atomics), so what is not arithmetic counts: block offsets are read four at a
-// time, nothing is staged.  12 MP chain frame, split products: stage 1 11.3 ->
-// 9.8 ms, stage 2 15.5 -> 13.0 ms against a form with a staging buffer, an
-// offset load per block and a scalar flush.
+// time, nothing is staged, the pairs of a segment overlap, and stage 1 keeps two
+// planes (64 registers: four CTAs an SM; stage 2 three).  12 MP chain frame, split
+// products: stage 1 11.3 -> 8.6 ms, stage 2 15.5 -> 12.5 ms against a form with a
+// staging buffer, an offset load and a branch per pair, and a scalar flush.  (The
+// products are not merged into MMAs of k = 16: another order of the sums moves
+// coefficients across the threshold.)
 template <int STAGE, bool SPLIT>
 __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int ty, int c, int img) {
     extern __shared__ __align__(16) float sm[];
@@ -900,9 +941,8 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* s_num = sm;
     float* s_img = sm + FP;                             // after the groups: the weight map, then den
-    float* s_bas = s_img + FP;                          // stage 2 (s_row at the flush)
-    float* s_row = s_img + FP;  // the footprint of the basic estimate in stage 2; at the flush the row-filtered map
-    float* s_wgt = s_row + FP;  // one aggregation weight per reference block of the tile
+    float* s_bas = s_img + FP;                          // stage 2: the basic estimate's footprint
+    float* s_wgt = s_img + (STAGE == 2 ? 2 : 1) * FP;   // one aggregation weight per reference block of the tile
     uint32_t* s_list = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_wgt + kRefTile * kRefTile) + 15) &
                                                    ~(uintptr_t)15);
     uint32_t* s_cnt = s_list + kRefTile * kRefTile * 16;
@@ -945,7 +985,7 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         int* woff = s_off + warp * 16;
         __syncwarp();
         if (lane < 16) {
-            const uint32_t p = lst[lane];
+            const uint32_t p = lst[lane < N ? lane : 0];
             woff[lane] = ((int)(p >> 16) - fy0) * P + (int)(p & 0xFFFFU) - fx0;
         }
         __syncwarp();
@@ -992,26 +1032,7 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
             wgt = sw2 > 0.0F ? 1.0F / fmaxf(sw2, kMinWienerEnergy) : a.sigma2;
         }
         if (lane == 0) s_wgt[k] = wgt;
-        float X[8][4];
-        tc_inverse<SPLIT>(H, N, dct, X);
-        // numerator, straight from the accumulators: an atomic instruction covers
-        // 8 columns x every other row of a block, 32 pixels in 32 banks (P = 4 mod 32)
-        const float kw0 = wgt * kq0, kw1 = wgt * kq1;
-        float* num = s_num + 2 * q * P + g;
-        int4 o = make_int4(0, 0, 0, 0);
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            if (2 * t >= N) break;
-            if (t % 2 == 0) o = *reinterpret_cast<const int4*>(woff + 2 * t);
-            float* d0 = num + (t % 2 ? o.z : o.x);
-            atomicAdd(d0, kw0 * X[t][0]);
-            atomicAdd(d0 + P, kw1 * X[t][1]);
-            if (2 * t + 1 < N) {
-                float* d1 = num + (t % 2 ? o.w : o.y);
-                atomicAdd(d1, kw0 * X[t][2]);
-                atomicAdd(d1 + P, kw1 * X[t][3]);
-            }
-        }
+        tc_inverse_add<SPLIT>(H, N, dct, wgt * kq0, wgt * kq1, s_num, P, woff);
     }
     __syncthreads();
     // weight map at the block origins (in the footprint's own plane, now free)
@@ -1028,35 +1049,37 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
     }
     __syncthreads();
     // den = map correlated with the Kaiser window (from the kernel arguments): rows
-    // into a free plane, then columns, four columns to a thread (16-byte loads);
-    // down the columns a thread keeps the last eight rows in registers
-    const int gx = (fw + 3) / 4;
-    for (int i = threadIdx.x; i < fh * gx; i += blockDim.x) {
-        const int yy = i / gx, xx = 4 * (i - yy * gx);
-        const float4* wr = reinterpret_cast<const float4*>(s_w + yy * P + xx);
-        const float4 w0 = xx >= 8 ? wr[-2] : zero4, w1 = xx >= 4 ? wr[-1] : zero4, w2 = wr[0];
-        const float w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
+    // in place, a band at a time, then columns, four columns to a thread (16-byte
+    // loads); down the columns a thread keeps the last eight rows in registers
+    const int gx = (fw + 3) / 4, segs = blockDim.x / gx;
+    const int seg = threadIdx.x / gx, xx = 4 * (threadIdx.x - seg * gx);
+    for (int b0 = 0; b0 < fh; b0 += segs) {
+        float4* wr = reinterpret_cast<float4*>(s_w + (b0 + seg) * P + xx);
+        const bool on = seg < segs && b0 + seg < fh;
         float h[4] = {0.0F, 0.0F, 0.0F, 0.0F};
+        if (on) {
+            const float4 w0 = xx >= 8 ? wr[-2] : zero4, w1 = xx >= 4 ? wr[-1] : zero4, w2 = wr[0];
+            const float w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < 8; ++u)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) h[k] = __fmaf_rn(a.kaiser1[u], w[8 + k - u], h[k]);
-        *reinterpret_cast<float4*>(s_row + yy * P + xx) = make_float4(h[0], h[1], h[2], h[3]);
+                for (int k = 0; k < 4; ++k) h[k] = __fmaf_rn(a.kaiser1[u], w[8 + k - u], h[k]);
+        }
+        __syncthreads();  // the band is read
+        if (on) *wr = make_float4(h[0], h[1], h[2], h[3]);
     }
     __syncthreads();
     float* gn = a.acc + (long long)c * a.npx;
     float* gd = a.acc + (long long)(3 + c) * a.npx;
-    const int segs = blockDim.x / gx, seg_rows = (fh + segs - 1) / segs;
-    for (int i = threadIdx.x; i < segs * gx; i += blockDim.x) {
-        const int seg = i / gx, xx = 4 * (i - seg * gx);
-        const int y0 = seg * seg_rows, y1 = min(fh, y0 + seg_rows);
-        if (y0 >= fh) continue;  // (more segments than rows)
-        float4 r[8];             // r[v]: the row v above
+    const int seg_rows = (fh + segs - 1) / segs;
+    const int y0 = seg * seg_rows, y1 = min(fh, y0 + seg_rows);
+    if (seg < segs && y0 < fh) {
+        float4 r[8];  // r[v]: the row v above
 #pragma unroll
         for (int v = 1; v < 8; ++v)
-            r[v] = y0 - v >= 0 ? *reinterpret_cast<const float4*>(s_row + (y0 - v) * P + xx) : zero4;
+            r[v] = y0 - v >= 0 ? *reinterpret_cast<const float4*>(s_w + (y0 - v) * P + xx) : zero4;
         for (int yy = y0; yy < y1; ++yy) {
-            r[0] = *reinterpret_cast<const float4*>(s_row + yy * P + xx);
+            r[0] = *reinterpret_cast<const float4*>(s_w + yy * P + xx);
             float4 d = zero4;
 #pragma unroll
             for (int v = 0; v < 8; ++v) {
@@ -1081,14 +1104,14 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
 }
 
 template <int STAGE, bool SPLIT>
-__global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_kernel(const __grid_constant__ FilterArgs a) {
+__global__ void __launch_bounds__(32 * kTcWarps, STAGE == 1 ? 4 : 3) bm3d_filter_tc_kernel(const __grid_constant__ FilterArgs a) {
     filter_tc_tile<STAGE, SPLIT>(a, blockIdx.x, blockIdx.y, blockIdx.z % 3, blockIdx.z / 3);
 }
 // A gated run seldom happens: a grid of resident CTAs that walk the tiles, so
 // that one which does not costs the launch (3 us) and not the start of every
 // tile's CTA (46 us a stage at 12 MP).
 template <int STAGE, bool SPLIT>
-__global__ void __launch_bounds__(32 * kTcWarps, 3) bm3d_filter_tc_gated_kernel(const __grid_constant__ FilterArgs a,
+__global__ void __launch_bounds__(32 * kTcWarps, STAGE == 1 ? 4 : 3) bm3d_filter_tc_gated_kernel(const __grid_constant__ FilterArgs a,
                                                                                int tiles) {
     if (gated_off(a.gate)) return;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -1176,9 +1199,9 @@ size_t match_layout(Bm3dPlan& p, int tile) {
 // 32 (column loads of eight columns x two rows, and atomics of eight rows x
 // four columns, fall in 32 different banks).
 int tile_pitch(int fw) { return fw + ((4 - fw) % 32 + 32) % 32; }
-size_t filter_tc_smem(const Bm3dPlan& p) {
+size_t filter_tc_smem(const Bm3dPlan& p, int stage) {
     const size_t fp = (size_t)p.fw * tile_pitch(p.fw);
-    const size_t floats = 3 * fp + kRefTile * kRefTile;  // numerator, two footprints, weights
+    const size_t floats = (stage == 2 ? 3 : 2) * fp + kRefTile * kRefTile;  // numerator, footprints, weights
     return sizeof(float) * floats + 16 + sizeof(uint32_t) * kRefTile * kRefTile * 17 + sizeof(int) * kTcWarps * 16;
 }
 
@@ -1263,16 +1286,16 @@ cudaError_t bm3d_setup(const Bm3dPlan& p) {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(bm3d_filter_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs2);
     if (p.tensor) {
-        const size_t ts = filter_tc_smem(p);
-        if (ts > kSmemOptIn) return cudaErrorInvalidConfiguration;
+        const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
+        if (ts2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
         const void* k1 = p.split ? (const void*)bm3d_filter_tc_kernel<1, true> : (const void*)bm3d_filter_tc_kernel<1, false>;
         const void* k2 = p.split ? (const void*)bm3d_filter_tc_kernel<2, true> : (const void*)bm3d_filter_tc_kernel<2, false>;
         const void* g1 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<1, true> : (const void*)bm3d_filter_tc_gated_kernel<1, false>;
         const void* g2 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<2, true> : (const void*)bm3d_filter_tc_gated_kernel<2, false>;
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts2);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts2);
     }
     return e;
 }
@@ -1296,7 +1319,7 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     cudaError_t e;
     if (setup && (e = bm3d_setup(p)) != cudaSuccess) return e;
     const size_t fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
-    const size_t ts = filter_tc_smem(p);
+    const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
 
     // a gated run's kernels walk the frame with few CTAs: it seldom happens, and
     // should not cost the start of a CTA for every row when it does not
@@ -1342,21 +1365,21 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
         ma.dthr = p.dthr[stage - 1];
         bm3d_match_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
         if (p.tensor && gate) {
-            const int tiles = p.ntx * p.nty * 3 * p.batch, g = std::min(tiles, kSmCount * 3);
+            const int tiles = p.ntx * p.nty * 3 * p.batch, g = std::min(tiles, kSmCount * (stage == 1 ? 4 : 3));
             if (p.split) {
-                if (stage == 1) bm3d_filter_tc_gated_kernel<1, true><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
-                else bm3d_filter_tc_gated_kernel<2, true><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, true><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, true><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
             } else {
-                if (stage == 1) bm3d_filter_tc_gated_kernel<1, false><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
-                else bm3d_filter_tc_gated_kernel<2, false><<<g, 32 * kTcWarps, ts, st>>>(ta, tiles);
+                if (stage == 1) bm3d_filter_tc_gated_kernel<1, false><<<g, 32 * kTcWarps, ts1, st>>>(ta, tiles);
+                else bm3d_filter_tc_gated_kernel<2, false><<<g, 32 * kTcWarps, ts2, st>>>(ta, tiles);
             }
         } else if (p.tensor) {
             if (p.split) {
-                if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
-                else bm3d_filter_tc_kernel<2, true><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
+                if (stage == 1) bm3d_filter_tc_kernel<1, true><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);
+                else bm3d_filter_tc_kernel<2, true><<<tgrid, 32 * kTcWarps, ts2, st>>>(ta);
             } else {
-                if (stage == 1) bm3d_filter_tc_kernel<1, false><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
-                else bm3d_filter_tc_kernel<2, false><<<tgrid, 32 * kTcWarps, ts, st>>>(ta);
+                if (stage == 1) bm3d_filter_tc_kernel<1, false><<<tgrid, 32 * kTcWarps, ts1, st>>>(ta);
+                else bm3d_filter_tc_kernel<2, false><<<tgrid, 32 * kTcWarps, ts2, st>>>(ta);
             }
         } else {
             for (int py = 0; py < p.phases; ++py)
