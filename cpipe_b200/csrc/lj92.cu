@@ -71,7 +71,8 @@ constexpr uint32_t kOverlapBits = 1536;  // bits decoded ahead of a chunk to syn
 constexpr int kChunksPerCta = 256;      // one chunk per thread; 8 groups of 32
 constexpr int kCands = 4;  // paths kept per chunk: lead, next phase, two from the exits of the chunk before
 constexpr int kGroupEntries = 2;  // group walks from a chunk group's lead path and its next-phase path
-constexpr int kStageWords = 8576;       // >= skewed words a CTA stages: (256 x 1024 + 1536 + 192) / 32 + 2 + skew
+constexpr uint32_t kStageSpan = (kChunksPerCta * kChunkBits + kOverlapBits + 192) / 32 + 2;  // words a CTA stages, at most
+constexpr int kStageWords = (kStageSpan + kStageSpan / 32 + 4) & ~3u;  // with the skew, a multiple of 16 bytes
 constexpr int kScanBytes = 4096;        // unstuff block: 256 threads x 16 bytes
 constexpr uint64_t kMaxParallelBytes = 1ull << 27;
 constexpr uint64_t kMaxParallelSamples = 1ull << 27;
@@ -120,26 +121,20 @@ struct CtaDesc {
 
 __device__ __forceinline__ uint32_t lj_tid(uint32_t tids, uint32_t ph) { return (tids >> (8 * ph)) & 0xFF; }
 
-// Most-significant-bit-first reader of an unstuffed stream of 32-bit words
-// [0, hi); words past it read as zero.  STAGED: words lo .. hi-1 held in
-// shared memory, already in big-endian order, word lo + r at r + r / 32 (one
-// skew word per 32 so that lanes reading chunks 32 words apart hit different
-// banks); otherwise the global stream.  After refill() the buffer holds at
-// least 33 bits, enough for one code and its extra bits.
-template <bool STAGED>
+// Most-significant-bit-first readers of an unstuffed stream of 32-bit words;
+// words past its end read as zero.  peek() gives the next 32 bits, enough for
+// one code and its extra bits (at most 16 + 15).
+
+// The global stream, by a bit buffer of up to 64 bits.
 struct LjBits {
     const uint32_t* w;
-    uint32_t lo, hi, next;
+    uint32_t hi, next;
     int nb;
     uint64_t buf;
-    uint4 q;         // global reader: the 16-byte line holding words qb .. qb+3 (the stream is 16-byte aligned
+    uint4 q;         // the 16-byte line holding words qb .. qb+3 (the stream is 16-byte aligned
     uint32_t qb;     // and zero-padded to a whole line past its end)
     __device__ __forceinline__ uint32_t word(uint32_t i) {
         if (i >= hi) return 0u;
-        if (STAGED) {
-            const uint32_t r = i - lo;
-            return w[r + (r >> 5)];
-        }
         if ((i & ~3u) != qb) {
             qb = i & ~3u;
             q = __ldg(reinterpret_cast<const uint4*>(w + qb));
@@ -152,61 +147,87 @@ struct LjBits {
         nb += 32;
         ++next;
     }
-    __device__ __forceinline__ void init(const uint32_t* words, uint32_t first, uint32_t end, uint32_t pos) {
+    __device__ __forceinline__ void init(const uint32_t* words, uint32_t end, uint32_t at) {
         w = words;
-        lo = first;
         hi = end;
         qb = 0xFFFFFFFFu;
-        next = pos >> 5;
+        next = at >> 5;
         buf = 0;
         nb = 0;
         refill();
         refill();
-        buf <<= (pos & 31);
-        nb -= (int)(pos & 31);
+        buf <<= (at & 31);
+        nb -= (int)(at & 31);
     }
     __device__ __forceinline__ uint32_t pos() const { return next * 32u - (uint32_t)nb; }
+    __device__ __forceinline__ uint32_t peek() {
+        if (nb <= 32) refill();
+        return (uint32_t)(buf >> 32);
+    }
+    __device__ __forceinline__ void skip(uint32_t n) {
+        buf <<= n;
+        nb -= (int)n;
+    }
 };
+
+// Words lo .. of the stream staged in shared memory, in big-endian order: word
+// lo + r at r + r / 32, and the first word of every 32 a second time in the slot
+// before it (lanes 32 words apart read from different banks, and a word's
+// successor always follows it).  The state is the bit position alone: a peek is
+// two loads and a funnel shift for every lane, where a bit buffer refills at
+// another step in each lane.
+struct LjWin {
+    const uint32_t* w;
+    uint32_t org;   // bit position of word lo
+    uint32_t last;  // reads start at word lo + last at most (two words of zeros past the stream)
+    uint32_t at;
+    __device__ __forceinline__ uint32_t pos() const { return at; }
+    // (kept inside the staged words by the caller's bound on `at`)
+    __device__ __forceinline__ uint32_t peek_at(uint32_t p) const {
+        const uint32_t r = (p - org) >> 5, k = r + (r >> 5);
+        return __funnelshift_l(w[k + 1], w[k], p);
+    }
+    __device__ __forceinline__ uint32_t peek() const {
+        const uint32_t r = min((at - org) >> 5, last), k = r + (r >> 5);
+        return __funnelshift_l(w[k + 1], w[k], at);
+    }
+    __device__ __forceinline__ void skip(uint32_t n) { at += n; }
+};
+
+// A code longer than kLutBits at the head of `w`: its length (up to 16), or 17
+// for an invalid one.
+__device__ __forceinline__ uint32_t lj_long(uint32_t w, const LjTab* tab, uint32_t& sym) {
+    uint32_t len = kLutBits + 1;
+    int code = (int)(w >> (32 - len));
+    while (len <= 16 && code > tab->maxcode[len]) {
+        ++len;
+        code = (int)(w >> (32 - len));
+    }
+    if (len <= 16) sym = tab->vals[tab->valoff[len] + code];
+    return len;
+}
 
 // One sample's difference, with the lookahead table `lut` and, for codes
 // longer than kLutBits, the canonical arrays of `tab`.  False on an invalid
 // code, after which the reader has consumed one bit (a deterministic step, so
 // paths from a wrong start still move on; on the true path it fails the
 // segment).
-template <class Bits>
-__device__ __forceinline__ bool lj_sym(Bits& br, const uint16_t* lut, const LjTab* tab, int& diff) {
-    if (br.nb <= 32) br.refill();
-    const uint32_t f = lut[(uint32_t)(br.buf >> (64 - kLutBits))];
-    int len, sym;
-    if (f) {
-        len = (int)((f >> 5) & 15u);
-        sym = (int)(f & 31u);
-    } else {
-        len = kLutBits + 1;
-        int code = (int)(br.buf >> (64 - len));
-        while (len <= 16 && code > tab->maxcode[len]) {
-            ++len;
-            code = (int)(br.buf >> (64 - len));
-        }
+__device__ __forceinline__ bool lj_sym(LjWin& br, const uint16_t* lut, const LjTab* tab, int& diff) {
+    const uint32_t w = br.peek();
+    const uint32_t f = lut[w >> (32 - kLutBits)];
+    uint32_t len = (f >> 5) & 15u, sym = f & 31u, total = f >> 9;
+    if (f == 0) {
+        len = lj_long(w, tab, sym);
         if (len > 16) {
-            br.buf <<= 1;
-            br.nb -= 1;
+            br.skip(1);
             return false;
         }
-        sym = tab->vals[tab->valoff[len] + code];
+        total = len + (sym < 16 ? sym : 0u);
     }
-    br.buf <<= len;
-    br.nb -= len;
-    if (sym == 0) {
-        diff = 0;
-    } else if (sym == 16) {
-        diff = 32768;
-    } else {
-        const int v = (int)(br.buf >> (64 - sym));
-        br.buf <<= sym;
-        br.nb -= sym;
-        diff = v < (1 << (sym - 1)) ? v - (1 << sym) + 1 : v;
-    }
+    br.skip(total);
+    const int v = (int)(((w << len) >> 1) >> (31 - sym));  // the sym extra bits (none for 0)
+    const int x = v < (int)((1u << sym) >> 1) ? v - (1 << sym) + 1 : v;
+    diff = sym == 16 ? 32768 : x;
     return true;
 }
 
@@ -214,7 +235,7 @@ __device__ __forceinline__ bool lj_sym(Bits& br, const uint16_t* lut, const LjTa
 struct LjCtx {
     const uint32_t* words;  // global stream
     uint32_t nw;            // its words
-    const uint32_t* sw;     // staged words lo .. hi-1 (kernels that stage)
+    const uint32_t* sw;     // staged words lo .. hi-1 (kernels that stage), zeros past the stream's end
     uint32_t lo, hi;
     uint32_t bits;          // stream length in bits (8 x unstuffed bytes)
     uint32_t last;          // last live chunk: the one holding the stream's final bit (0 for an empty stream)
@@ -225,84 +246,138 @@ struct LjCtx {
     __device__ __forceinline__ uint32_t step(uint32_t ph) const { return shared ? 0u : (ph + 1 == nf ? 0u : ph + 1); }
     __device__ __forceinline__ uint32_t cs(uint32_t c) const { return c * kChunkBits; }
     __device__ __forceinline__ uint32_t ce(uint32_t c) const { return c >= last ? bits : (c + 1) * kChunkBits; }
-    template <bool STAGED>
-    __device__ __forceinline__ void open(LjBits<STAGED>& br, uint32_t pos) const {
-        if (STAGED) br.init(sw, lo, hi, pos);
-        else br.init(words, 0, nw, pos);
+    __device__ __forceinline__ void open(LjBits& br, uint32_t pos) const { br.init(words, nw, pos); }
+    __device__ __forceinline__ void open(LjWin& br, uint32_t pos) const {
+        br.w = sw;
+        br.org = lo * 32u;
+        br.last = hi - lo - 2u;
+        br.at = pos;
     }
 };
 
-template <class Bits>
-__device__ __forceinline__ bool lj_next(const LjCtx& x, Bits& br, uint32_t ph, int& diff) {
+// Run tables, one per phase, over the next kLutBits bits: what a reader in that
+// phase may skip at once.  A flat stretch (clipped lights, the padding of an edge
+// tile) codes a sample in one or two bits, and a chunk of it would be a chain of a
+// thousand lookups.  6 MP of 10-bit tiles, a table per component: lj_cand_kernel
+// 268 -> 108 us, lj_write_kernel 105 -> 61 us against a bit buffer a lane and a
+// sample a lookup (169 and 72 us with the position-only reader alone).
+// Counting paths: the samples that lie whole in the window, or the first one if
+// none does.
+//   bits 0-4 their length, 5-8 their count, 9-10 the phase after them, 11-15 the
+//   length of the first; 0 where the first code is longer than the window
+__device__ __forceinline__ uint32_t run_entry(const uint16_t* lut, uint32_t nf, uint32_t ph, uint32_t idx) {
+    const uint32_t f0 = lut[ph * kLut + idx] >> 9;
+    if (f0 == 0) return 0;
+    uint32_t at = f0, n = 1, p = ph + 1 == nf ? 0u : ph + 1;
+    while (at < kLutBits) {
+        // (the bits past the window read as zeros: an entry counts if it needs none of them)
+        const uint32_t f = lut[p * kLut + ((idx << at) & (kLut - 1))] >> 9;
+        if (f == 0 || at + f > kLutBits) break;
+        at += f;
+        ++n;
+        p = p + 1 == nf ? 0u : p + 1;
+    }
+    return at | (n << 5) | (p << 9) | (f0 << 11);
+}
+// Writing: the leading samples of difference 0, in fours.
+//   bits 0-3 their length, 4-5 the phase after them, 6-7 fours
+__device__ __forceinline__ uint32_t zero_entry(const uint16_t* lut, uint32_t nf, uint32_t ph, uint32_t idx) {
+    uint32_t at = 0, n = 0, p = ph, e = 0;
+    while (at < kLutBits) {
+        const uint32_t f = lut[p * kLut + ((idx << at) & (kLut - 1))];
+        if (f == 0 || (f & 31u) != 0 || at + (f >> 9) > kLutBits) break;
+        at += f >> 9;
+        p = p + 1 == nf ? 0u : p + 1;
+        if ((++n & 3u) == 0) e = at | (p << 4) | ((n / 4) << 6);
+    }
+    return e;
+}
+
+__device__ __forceinline__ bool lj_next(const LjCtx& x, LjWin& br, uint32_t ph, int& diff) {
     const uint32_t tp = x.shared ? 0u : ph;
     return lj_sym(br, x.lut + tp * kLut, x.tabs + lj_tid(x.tids, tp), diff);
 }
 
-// Skips one sample's code and extra bits (counting paths need no values).
-// False on an invalid code, after which one bit is consumed, as in lj_sym.
-template <class Bits>
-__device__ __forceinline__ bool lj_skip(Bits& br, const uint16_t* lut, const LjTab* tab) {
-    if (br.nb <= 32) br.refill();
-    const uint32_t f = lut[(uint32_t)(br.buf >> (64 - kLutBits))];
-    int total;
-    if (f) {
-        total = (int)(f >> 9);
-    } else {
-        int len = kLutBits + 1;
-        int code = (int)(br.buf >> (64 - len));
-        while (len <= 16 && code > tab->maxcode[len]) {
-            ++len;
-            code = (int)(br.buf >> (64 - len));
-        }
-        if (len > 16) {
-            br.buf <<= 1;
-            br.nb -= 1;
-            return false;
-        }
-        const int sym = tab->vals[tab->valoff[len] + code];
-        total = len + (sym < 16 ? sym : 0);
-    }
-    br.buf <<= total;
-    br.nb -= total;
-    return true;
+// Bits of the sample at the head of `w` (counting paths need no values), given
+// its lookahead entry f; `ok` is cleared on an invalid code, of which one bit is
+// consumed, as in lj_sym.
+__device__ __forceinline__ uint32_t lj_total(const LjCtx& x, uint32_t w, uint32_t f, uint32_t ph, bool& ok) {
+    if (f) return f >> 9;
+    uint32_t sym = 0;
+    const uint32_t len = lj_long(w, x.tabs + lj_tid(x.tids, ph), sym);
+    ok = len <= 16;
+    return ok ? len + (sym < 16 ? sym : 0u) : 1u;
 }
 
 // From (pos, ph): to the first sample boundary at or after cs (the start
-// state), then to the first at or after ce (the exit), counting samples.
-// SHARED: one table, the phase stays 0.
-template <bool STAGED, bool SHARED>
-__device__ __forceinline__ LjCand lj_path_t(const LjCtx& x, uint32_t pos, uint32_t ph, uint32_t cs, uint32_t ce) {
-    LjBits<STAGED> br;
+// state), then to the first at or after ce (the exit), counting samples.  A
+// sample at a time (the walks, where a chunk did not synchronise).
+template <class Bits>
+__device__ __forceinline__ LjCand lj_path(const LjCtx& x, uint32_t pos, uint32_t ph, uint32_t cs, uint32_t ce) {
+    Bits br;
     x.open(br, pos);
-    const LjTab* tab0 = x.tabs + lj_tid(x.tids, 0);
-    while (br.pos() < cs) {
-        if (SHARED) {
-            lj_skip(br, x.lut, tab0);
-        } else if (lj_skip(br, x.lut + ph * kLut, x.tabs + lj_tid(x.tids, ph))) {
-            ph = ph + 1 == x.nf ? 0u : ph + 1;
-        }
-    }
+    auto next = [&]() {
+        const uint32_t w = br.peek();
+        bool ok = true;
+        br.skip(lj_total(x, w, x.lut[ph * kLut + (w >> (32 - kLutBits))], ph, ok));
+        if (ok) ph = x.step(ph);
+        return (uint32_t)ok;
+    };
+    while (br.pos() < cs) next();
     LjCand c;
     c.s = br.pos();
     const uint32_t sp = ph;
     uint32_t n = 0;
-    while (br.pos() < ce) {
-        if (SHARED) {
-            n += lj_skip(br, x.lut, tab0);
-        } else if (lj_skip(br, x.lut + ph * kLut, x.tabs + lj_tid(x.tids, ph))) {
-            ph = ph + 1 == x.nf ? 0u : ph + 1;
-            ++n;
-        }
-    }
+    while (br.pos() < ce) n += next();
     c.e = br.pos();
     c.n = n;
     c.meta = sp | (ph << 2) | 16u;
     return c;
 }
 
-template <bool STAGED>
-__device__ __forceinline__ LjCand lj_path(const LjCtx& x, uint32_t pos, uint32_t ph, uint32_t cs, uint32_t ce) {
-    return x.shared ? lj_path_t<STAGED, true>(x, pos, 0, cs, ce) : lj_path_t<STAGED, false>(x, pos, ph, cs, ce);
+// A path over the staged words, by the run tables `runs` (lj_cand_kernel): a
+// window at a time while one fits before the limit, then a sample at a time.
+struct LjRun {
+    uint32_t pos, ph, n;
+    __device__ __forceinline__ void step(const LjCtx& x, const uint16_t* runs, const LjWin& br, bool whole, bool on = true) {
+        const uint32_t w = br.peek_at(pos);
+        const uint32_t f = runs[ph * kLut + (w >> (32 - kLutBits))];
+        uint32_t total = whole ? f & 31u : f >> 11, count = whole ? (f >> 5) & 15u : 1u;
+        uint32_t after = whole ? (f >> 9) & 3u : x.step(ph);
+        if (f == 0) {
+            bool ok = true;
+            total = lj_total(x, w, 0, ph, ok);
+            count = ok;
+            after = ok ? x.step(ph) : ph;
+        }
+        if (on) {
+            pos += total;
+            n += count;
+            ph = after;
+        }
+    }
+    __device__ __forceinline__ void to(const LjCtx& x, const uint16_t* runs, const LjWin& br, uint32_t lim) {
+        while (pos + kLutBits <= lim) step(x, runs, br, true);
+        while (pos < lim) step(x, runs, br, false);
+    }
+};
+
+// Two paths to the limit side by side, as each is a chain of dependent loads.
+__device__ __forceinline__ void lj_run_pair(const LjCtx& x, const uint16_t* runs, const LjWin& br, uint32_t lim, LjRun& a,
+                                            LjRun& b) {
+    while (a.pos + kLutBits <= lim || b.pos + kLutBits <= lim) {
+        a.step(x, runs, br, true, a.pos + kLutBits <= lim);
+        b.step(x, runs, br, true, b.pos + kLutBits <= lim);
+    }
+    while (a.pos < lim || b.pos < lim) {
+        // (a path past the limit stands less than a sample past it: its loads stay inside the staged words)
+        a.step(x, runs, br, false, a.pos < lim);
+        b.step(x, runs, br, false, b.pos < lim);
+    }
+}
+
+__device__ __forceinline__ LjCand lj_cand(const LjRun& from, const LjRun& to) {
+    return LjCand{from.pos, to.pos, to.n, from.ph | (to.ph << 2) | 16u};
 }
 
 // The lookahead tables of the segment's phases into shared memory, 16 bytes a
@@ -347,19 +422,23 @@ __device__ __forceinline__ LjCtx make_ctx(const SegDev& s, const uint8_t* ubuf, 
 }
 
 // Words a CTA over chunks c0 .. c0 + kChunksPerCta - 1 reads: from its first
-// chunk's lead to past its last live chunk's exit and the reader's lookahead.
+// chunk's lead to past its last live chunk's exit and the reader's lookahead
+// (at least two words past that chunk's last bit).
 __device__ __forceinline__ void stage_range(const LjCtx& x, uint32_t c0, uint32_t* lo, uint32_t* hi) {
     const uint32_t cs0 = x.cs(c0), lead = kOverlapBits;
     *lo = (cs0 > lead ? cs0 - lead : 0) >> 5;
     const uint32_t cl = min(c0 + kChunksPerCta - 1, x.last);
-    *hi = min(x.nw, (x.ce(cl) + 192) / 32 + 1);
-    if (*hi < *lo) *hi = *lo;
+    *hi = (x.ce(cl) + 192) / 32 + 1;
+    if (*hi < *lo + 2) *hi = *lo + 2;  // (a CTA past the stream's end)
 }
 
-// Byte-swapped, skewed copy of words lo .. hi-1 into shared memory.
+// Byte-swapped, skewed copy of words lo .. hi-1 into shared memory (LjWin).
 __device__ __forceinline__ void stage_words(uint32_t* sw, const LjCtx& x, uint32_t lo, uint32_t hi) {
-    for (uint32_t r = threadIdx.x; r < hi - lo; r += blockDim.x)
-        sw[r + (r >> 5)] = __byte_perm(__ldg(x.words + lo + r), 0, 0x0123);
+    for (uint32_t r = threadIdx.x; r < hi - lo; r += blockDim.x) {
+        const uint32_t v = lo + r < x.nw ? __byte_perm(__ldg(x.words + lo + r), 0, 0x0123) : 0u;
+        sw[r + (r >> 5)] = v;
+        if ((r & 31u) == 0 && r > 0) sw[r + (r >> 5) - 1] = v;
+    }
 }
 
 // ---------------------------------------------------------------- unstuffing
@@ -482,18 +561,12 @@ __global__ void __launch_bounds__(256) lj_pack_kernel(const uint8_t* __restrict_
 }
 
 // ------------------------------------------------------ candidates and walks
-// Shared memory of the staging kernels: the lookahead tables of the
-// segment's phases, then its staged words.
-__device__ __forceinline__ LjCtx open_cta(const SegDev& s, const uint8_t* ubuf, uint32_t ulen, const LjTab* tabs,
-                                          uint32_t c0, uint32_t* smem) {
-    uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
-    uint32_t* sw = smem + (s.shared ? 1u : s.nf) * (kLut / 2);  // after the phases' tables
-    stage_luts(lut, tabs, s);
+// Context of the kernels that stage: tables at `lut`, words at `sw`, both still to be filled.
+__device__ __forceinline__ LjCtx staged_ctx(const SegDev& s, const uint8_t* ubuf, uint32_t ulen, const LjTab* tabs,
+                                            uint32_t c0, const uint16_t* lut, const uint32_t* sw) {
     LjCtx x = make_ctx(s, ubuf, ulen, lut, tabs);
     stage_range(x, c0, &x.lo, &x.hi);
-    stage_words(sw, x, x.lo, x.hi);
     x.sw = sw;
-    __syncthreads();
     return x;
 }
 
@@ -507,10 +580,24 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_cand_kernel(const SegDev* __
                                                                 LjCand* __restrict__ cand) {
     const CtaDesc d = ctas[blockIdx.x];
     const SegDev s = segs[d.seg];
-    uint32_t* smem = reinterpret_cast<uint32_t*>(lj_dyn_smem);
-    const LjCtx x = open_cta(s, ubuf, ulen[d.seg], tabs, d.c0, smem);
-    // this CTA's first paths, after the tables and the staged words
-    LjCand* first = reinterpret_cast<LjCand*>(smem + (s.shared ? 1u : s.nf) * (kLut / 2) + kStageWords);
+    // the run tables, the staged words (first the lookahead tables, for the run
+    // tables to be made from), this CTA's first paths
+    const uint32_t phases = s.shared ? 1u : s.nf;
+    uint16_t* runs = reinterpret_cast<uint16_t*>(lj_dyn_smem);
+    uint32_t* sw = reinterpret_cast<uint32_t*>(lj_dyn_smem) + phases * (kLut / 2);
+    LjCand* first = reinterpret_cast<LjCand*>(sw + kStageWords);
+    uint16_t* lut = reinterpret_cast<uint16_t*>(sw);
+    static_assert(kStageWords * 4 >= 4 * kLut * 2, "the lookahead tables fit where the words go");
+    const LjCtx x = staged_ctx(s, ubuf, ulen[d.seg], tabs, d.c0, lut, sw);
+    stage_luts(lut, tabs, s);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < phases * kLut; i += blockDim.x)
+        runs[i] = (uint16_t)run_entry(lut, phases, i / kLut, i % kLut);
+    __syncthreads();
+    stage_words(sw, x, x.lo, x.hi);
+    __syncthreads();
+    LjWin br;
+    x.open(br, 0);
     const uint32_t c = d.c0 + threadIdx.x;
     const bool live = c < s.nchunk && c <= x.last;
     const LjCand none = {0, 0, 0, 0};
@@ -518,12 +605,19 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_cand_kernel(const SegDev* __
     LjCand p0 = none, p1 = none;
     if (live) {
         // the stream's start is exact; elsewhere a lead of kOverlapBits
-        p0 = lj_path<true>(x, c == 0 ? 0 : (cs > kOverlapBits ? cs - kOverlapBits : 0), 0, cs, ce);
-        // Different tables per component: the same start one phase on.  Where
-        // the tables give the codes in play the same lengths (a flat stretch, a
-        // padded tile edge) a path can sit on the true boundaries one
+        LjRun a = {cs > kOverlapBits ? cs - kOverlapBits : 0, 0, 0};
+        a.to(x, runs, br, cs);
+        a.n = 0;
+        // Different tables per component: also the same start one phase on.
+        // Where the tables give the codes in play the same lengths (a flat
+        // stretch, a padded tile edge) a path can sit on the true boundaries one
         // component off for any length.
-        if (c > 0 && !x.shared) p1 = lj_path<true>(x, p0.s, ((p0.meta & 3u) + 1) % x.nf, cs, ce);
+        const bool two = c > 0 && !x.shared;
+        LjRun b = {two ? a.pos : ce, x.step(a.ph), 0};
+        const LjRun a0 = a, b0 = b;
+        lj_run_pair(x, runs, br, ce, a, b);
+        p0 = lj_cand(a0, a);
+        if (two) p1 = lj_cand(b0, b);
     }
     first[2 * threadIdx.x] = p0;
     first[2 * threadIdx.x + 1] = p1;
@@ -531,37 +625,34 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_cand_kernel(const SegDev* __
     // Where a path of the chunk before leaves at a state that starts none of
     // this chunk's paths, one more path from that exact state: the walks then
     // miss only where neighbouring chunks both failed to synchronise.
+    // A second round does the same over the paths the first one added, for runs
+    // of two chunks that did not synchronise.
     LjCand f0 = none, f1 = none;
-    if (live && c > 0 && threadIdx.x > 0)
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+        if (live && c > 0 && threadIdx.x > 0)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const LjCand q = first[2 * (threadIdx.x - 1) + j];
-            const uint32_t ep = (q.meta >> 2) & 3u;
-            auto starts = [&](const LjCand& r) { return (r.meta & 16u) && r.s == q.e && (r.meta & 3u) == ep; };
-            if ((q.meta & 16u) && !starts(p0) && !starts(p1) && !starts(f0)) {
-                const LjCand r = lj_path<true>(x, q.e, ep, cs, ce);
-                if (f0.meta & 16u) f1 = r;
-                else f0 = r;
+            for (int j = 0; j < 2; ++j) {
+                const LjCand q = first[2 * (threadIdx.x - 1) + j];
+                const LjRun at = {q.e, (q.meta >> 2) & 3u, 0};
+                auto starts = [&](const LjCand& r) {
+                    return (r.meta & 16u) && r.s == at.pos && (r.meta & 3u) == at.ph;
+                };
+                if ((q.meta & 16u) && !(f1.meta & 16u) && !starts(p0) && !starts(p1) && !starts(f0)) {
+                    LjRun a = at;
+                    a.to(x, runs, br, ce);
+                    const LjCand r = lj_cand(at, a);
+                    if (f0.meta & 16u) f1 = r;
+                    else f0 = r;
+                }
             }
+        if (round == 0) {
+            __syncthreads();
+            first[2 * threadIdx.x] = f0;
+            first[2 * threadIdx.x + 1] = f1;
+            __syncthreads();
         }
-    // A second round over the paths the first one added, for runs of two
-    // chunks that did not synchronise.
-    __syncthreads();
-    first[2 * threadIdx.x] = f0;
-    first[2 * threadIdx.x + 1] = f1;
-    __syncthreads();
-    if (live && c > 0 && threadIdx.x > 0 && !(f1.meta & 16u))
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const LjCand q = first[2 * (threadIdx.x - 1) + j];
-            const uint32_t ep = (q.meta >> 2) & 3u;
-            auto starts = [&](const LjCand& r) { return (r.meta & 16u) && r.s == q.e && (r.meta & 3u) == ep; };
-            if ((q.meta & 16u) && !(f1.meta & 16u) && !starts(p0) && !starts(p1) && !starts(f0)) {
-                const LjCand r = lj_path<true>(x, q.e, ep, cs, ce);
-                if (f0.meta & 16u) f1 = r;
-                else f0 = r;
-            }
-        }
+    }
     if (c >= s.nchunk) return;
     LjCand* out = cand + (size_t)(s.chunk0 + c) * kCands;
     out[0] = p0;
@@ -576,7 +667,7 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_cand_kernel(const SegDev* __
 // that exact state (or, with give_up, the walk returns false there).  On
 // return (pos, ph) is the group's exit, `total` has grown by its samples, and
 // lane j holds its chunk's exact start and count.
-template <bool STAGED>
+template <class Bits>
 __device__ bool lj_walk(const LjCtx& x, const LjCand (&c)[kCands], uint32_t gc0, uint32_t glive, uint32_t& pos,
                         uint32_t& ph, uint32_t& my_pos, uint32_t& my_ph, uint32_t& my_n, uint32_t& total,
                         unsigned long long* stats, int which, bool give_up = false) {
@@ -595,7 +686,7 @@ __device__ bool lj_walk(const LjCtx& x, const LjCand (&c)[kCands], uint32_t gc0,
                 }
             if (!hit && !give_up) {
                 const uint32_t cc = gc0 + j;
-                const LjCand r = lj_path<STAGED>(x, pos, ph, x.cs(cc), x.ce(cc));
+                const LjCand r = lj_path<Bits>(x, pos, ph, x.cs(cc), x.ce(cc));
                 e = r.e;
                 ep = (r.meta >> 2) & 3u;
                 n = r.n;
@@ -667,7 +758,7 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_group_kernel(const SegDev* _
             uint32_t mp = 0, mph = 0, mn = 0, total = 0;
             // the lead path's walk decodes missing chunks again; the other
             // phase's walk gives up at its first miss
-            if (lj_walk<false>(x, c, gc0, glive, pos, ph, mp, mph, mn, total, stats, kStatGroup, k > 0))
+            if (lj_walk<LjBits>(x, c, gc0, glive, pos, ph, mp, mph, mn, total, stats, kStatGroup, k > 0))
                 g = LjGroup{s0, pos, total, p0 | (ph << 2) | 16u};
         }
         if (lane == 0) out[k] = g;
@@ -718,7 +809,7 @@ __global__ void __launch_bounds__(32) lj_seg_kernel(const SegDev* __restrict__ s
                 load_cands(cand, s, gc0, glive, c);
                 uint32_t mp = 0, mph = 0, mn = 0;
                 if (lane == 0) atomicAdd(stats + kStatGroupMiss, 1ull);
-                lj_walk<false>(x, c, gc0, glive, pos, ph, mp, mph, mn, off, stats, kStatSeg);
+                lj_walk<LjBits>(x, c, gc0, glive, pos, ph, mp, mph, mn, off, stats, kStatSeg);
             }
         }
     }
@@ -737,7 +828,18 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_write_kernel(const SegDev* _
                                                                  unsigned long long* stats) {
     const CtaDesc d = ctas[blockIdx.x];
     const SegDev s = segs[d.seg];
-    const LjCtx x = open_cta(s, ubuf, ulen[d.seg], tabs, d.c0, reinterpret_cast<uint32_t*>(lj_dyn_smem));
+    // the lookahead tables, the staged words, the tables of zero runs
+    const uint32_t phases = s.shared ? 1u : s.nf;
+    uint16_t* lut = reinterpret_cast<uint16_t*>(lj_dyn_smem);
+    uint32_t* sw = reinterpret_cast<uint32_t*>(lj_dyn_smem) + phases * (kLut / 2);
+    uint8_t* zeros = reinterpret_cast<uint8_t*>(sw + kStageWords);
+    const LjCtx x = staged_ctx(s, ubuf, ulen[d.seg], tabs, d.c0, lut, sw);
+    stage_luts(lut, tabs, s);
+    stage_words(sw, x, x.lo, x.hi);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < phases * kLut; i += blockDim.x)
+        zeros[i] = (uint8_t)zero_entry(lut, phases, i / kLut, i % kLut);
+    __syncthreads();
     const uint32_t gc0 = d.c0 + (threadIdx.x >> 5) * 32;
     if (gc0 >= s.nchunk || gc0 > x.last) return;  // warp-uniform
     const uint32_t lane = threadIdx.x & 31;
@@ -746,7 +848,7 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_write_kernel(const SegDev* _
     LjCand c[kCands];
     load_cands(cand, s, gc0, glive, c);
     uint32_t pos = ge.x, ph = ge.y, total = 0, my_pos = 0, my_ph = 0, my_n = 0;
-    lj_walk<true>(x, c, gc0, glive, pos, ph, my_pos, my_ph, my_n, total, stats, kStatWrite);
+    lj_walk<LjWin>(x, c, gc0, glive, pos, ph, my_pos, my_ph, my_n, total, stats, kStatWrite);
     uint32_t inc = lane < glive ? my_n : 0;
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
@@ -758,7 +860,7 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_write_kernel(const SegDev* _
     // the stream's last chunk goes on (through zeros past a short stream) to the frame's last sample
     const uint32_t lim = gc0 + lane == x.last ? samples : min(t0 + my_n, samples);
     if (t0 >= lim) return;
-    LjBits<true> br;
+    LjWin br;
     x.open(br, my_pos);
     uint16_t* o = dbuf + s.sbase;  // 8-byte aligned: segments start on a multiple of 4 samples
     uint32_t p = my_ph, t = t0;
@@ -771,7 +873,15 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_write_kernel(const SegDev* _
         }
         o[t] = (uint16_t)diff;
     }
-    for (; t + 4 <= lim; t += 4) {
+    while (t + 4 <= lim) {
+        const uint32_t z = zeros[p * kLut + (br.peek() >> (32 - kLutBits))], run = 4u * (z >> 6);
+        if (run && t + run <= lim) {
+            for (uint32_t k = 0; k < run; k += 4) *reinterpret_cast<uint64_t*>(o + t + k) = 0;
+            t += run;
+            p = (z >> 4) & 3u;
+            br.skip(z & 15u);
+            continue;
+        }
         uint64_t four = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k, p = x.step(p)) {
@@ -782,6 +892,7 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_write_kernel(const SegDev* _
             four |= (uint64_t)(uint16_t)diff << (16 * k);
         }
         *reinterpret_cast<uint64_t*>(o + t) = four;
+        t += 4;
     }
     for (; t < lim; ++t, p = x.step(p)) {
         if (!lj_next(x, br, p, diff)) {
@@ -1349,22 +1460,25 @@ int lj92_decode(const uint8_t* const* streams, const size_t* bytes, uint32_t cou
                                                                   static_cast<const uint32_t*>(d_boff), ubuf, ulen);
         }
         // per call: the attribute belongs to the current device
-        const int most = 4 * kLut * 2 + kStageWords * 4 + kChunksPerCta * 2 * (int)sizeof(LjCand);
+        // (and always the most that any file takes, so that concurrent calls agree on it)
+        auto cand_smem = [](uint32_t phases) {
+            return (int)(phases * kLut * 2 + kStageWords * 4 + kChunksPerCta * 2 * sizeof(LjCand));
+        };
+        auto write_smem = [](uint32_t phases) { return (int)(phases * kLut * 3 + kStageWords * 4); };
         const bool attrs =
-            cudaFuncSetAttribute(lj_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
-            cudaFuncSetAttribute(lj_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+            cudaFuncSetAttribute(lj_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cand_smem(4)) == cudaSuccess &&
+            cudaFuncSetAttribute(lj_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, write_smem(4)) == cudaSuccess;
         if (!attrs) {
             cudaGetLastError();
             set_error("%s", "lj92: shared memory attribute refused");
             return call.finish(CPIPE_INTERNAL_ERROR);
         }
-        const size_t smem = (size_t)max_phases * kLut * 2 + kStageWords * 4;
-        lj_cand_kernel<<<nctas, kChunksPerCta, smem + kChunksPerCta * 2 * sizeof(LjCand), call.stream>>>(
+        lj_cand_kernel<<<nctas, kChunksPerCta, cand_smem(max_phases), call.stream>>>(
             dsegs, dctas, dtabs, ubuf, ulen, cand);
         lj_group_kernel<<<nctas, kChunksPerCta, 0, call.stream>>>(dsegs, dctas, dtabs, ubuf, ulen, cand, grp,
                                                                   dstats);
         lj_seg_kernel<<<npar, 32, 0, call.stream>>>(dsegs, dpar, dtabs, ubuf, ulen, cand, grp, gentry, dstats);
-        lj_write_kernel<<<nctas, kChunksPerCta, smem, call.stream>>>(dsegs, dctas, dtabs, ubuf, ulen, cand, gentry, dbuf,
+        lj_write_kernel<<<nctas, kChunksPerCta, write_smem(max_phases), call.stream>>>(dsegs, dctas, dtabs, ubuf, ulen, cand, gentry, dbuf,
                                                                   dstatus, dstats);
         if (!lines.empty()) {
             lj_col_kernel<<<npar, 32, 0, call.stream>>>(dsegs, dpar, dbuf, cbuf);

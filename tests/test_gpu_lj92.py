@@ -219,3 +219,26 @@ def test_subifd_files(cuda_device):
     st, got = dng_decode(subifd_dng(flat), 70, 48)
     assert st == 0, A.lib().cpipe_cuda_last_error()
     np.testing.assert_array_equal(got, img)
+
+
+@pytest.mark.parametrize("tables", ["fixed", "per_component"])
+@pytest.mark.parametrize("nf", [1, 2, 3, 4])
+def test_flat_runs(cuda_device, nf, tables):
+    """Runs of equal samples of every length around the lookahead window's (12
+    samples of one-bit codes) between noise, whole flat lines, and a frame that
+    ends flat: a chunk of them holds far more samples than one of noise."""
+    from cpipe_b200.dng_synth import lj92_segment
+    rng = np.random.default_rng(nf)
+    w = 96 * nf
+    img = np.repeat(rng.integers(0, 1024, (200, 1)), w, 1)
+    for y in range(0, 140, 2):
+        x = 0
+        while x < w:  # runs of 1 .. 29 samples, then 1 .. 5 noisy ones
+            n, m = int(rng.integers(1, 30)), int(rng.integers(1, 6))
+            img[y, x:x + m] = rng.integers(0, 1024, img[y, x:x + m].size)
+            x += n + m
+    img = img.astype(np.uint16)
+    st, got = gpu_decode([lj92_segment(img, 10, nf, tables)], 1, w, 200, w, 200)
+    assert st == 0, A.lib().cpipe_cuda_last_error()
+    np.testing.assert_array_equal(got, img)
+    assert _stats()[2:] == (1, 0)
