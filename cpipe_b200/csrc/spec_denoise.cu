@@ -72,15 +72,22 @@ namespace {
 //        same way; per pixel
 //        out = max(mean_a v + mean_b, 0) (means as products with 1/N) held in
 //        registers, then written with the input's alpha.
+// ab is bound by issue, out by shared-memory bandwidth and the wait for its
+// copies, so both read a window's leaving values once (held in registers from
+// the first sum), put the row windows on whole warps, copy a row with columns
+// clamped once a block, and out fetches the next channel under the column pass:
+// 12 MP binary16, R = 8: ab 184 -> 158 us, out 207 -> 184 us.
 // Each running sum adds at most 2R+1 + 2 * 15 terms, so binary16 frames stay
 // within one binary16 ulp of the FP64 definition and binary32 frames within
 // 1e-5.  Shared-memory pitches are odd (in elements of the stored type), so
 // the lanes of a warp (rows in the row pass, columns in the column pass) hit
 // distinct banks.
 constexpr int kGsTW = 64, kGsTH = 32, kGsRunX = 16, kGsRunY = 8, kGsThreads = 256;
+constexpr int kGsKeepOut = 7;  // (all 15 would spill beside the pixels and results held)
+constexpr int kGsCols = (kGsTW + 2 * kGuidedSpecMaxRadius + 31) / 32;  // staged columns a lane copies, at most
 static_assert(kGsTW * (kGsTH / kGsRunY) == kGsThreads, "one column window per thread");
 static_assert((kGsTW / kGsRunX) * 64 == kGsThreads && kGsTH + 2 * kGuidedSpecMaxRadius <= 64,
-              "one row window per thread: the staged rows fit 64 lanes");
+              "at most one row window per thread");
 struct GsPlanes {
     int w, h, R, Wa, Ha;
     float* a;  // [3][Ha][Wa]
@@ -101,7 +108,28 @@ __host__ __device__ constexpr size_t gs_ab_smem(int R) {
 __host__ __device__ constexpr size_t gs_out_smem(int R) {
     return (size_t)(kGsTH + 2 * R) * gs_pitch(R) * 8 + (size_t)(kGsTH + 2 * R) * kGsPH * 8;
 }
-__device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }
+// a - b, both at once (the product with -1 is exact)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0F, -1.0F), a); }
+// RUN sliding sums over D values: load(k) is the k-th value of the first window,
+// store(i, sum) takes the i-th window's.  The first KEEP values are held in
+// registers for their second use (load must be valid below KEEP + RUN for any D).
+template <int RUN, int KEEP, class Load, class Store>
+__device__ __forceinline__ void gs_slide(int D, Load load, Store store) {
+    float2 held[KEEP], s = make_float2(0.0F, 0.0F);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        held[k] = load(k);
+        if (k < D) s = __fadd2_rn(s, held[k]);
+    }
+#pragma unroll 4
+    for (int k = KEEP; k < D; ++k) s = __fadd2_rn(s, load(k));
+    store(0, s);
+#pragma unroll
+    for (int i = 1; i < RUN; ++i) {
+        s = sub2(__fadd2_rn(s, load(i + D - 1)), i - 1 < KEEP ? held[i - 1 < KEEP ? i - 1 : 0] : load(i - 1));
+        store(i, s);
+    }
+}
 // 4-byte asynchronous global -> shared copies: a warp's whole staging is in
 // flight at once instead of one dependent load per iteration.
 __device__ __forceinline__ void gs_cp4(void* dst, const void* src) {
@@ -117,7 +145,7 @@ template <>
 __device__ __forceinline__ float gs_val<float>(uint32_t word, int) { return __uint_as_float(word); }
 template <>
 __device__ __forceinline__ float gs_val<__half>(uint32_t word, int c) {
-    return __half2float(__ushort_as_half((unsigned short)((c & 1) ? (word >> 16) : (word & 0xFFFFU))));
+    return __half2float(__ushort_as_half((unsigned short)__byte_perm(word, 0, (c & 1) ? 0x32 : 0x10)));
 }
 
 template <class T>
@@ -131,60 +159,52 @@ __global__ void __launch_bounds__(kGsThreads) gsp_ab_kernel(Img in, GsPlanes p, 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // plane column X0 + q's box starts at image column X0 - 2R + q
     const int cw = std::is_same<T, float>::value ? c : (c & ~1);  // element of the staged word
+    unsigned col[kGsCols];  // the lane's columns, the same in every row
+#pragma unroll
+    for (int j = 0; j < kGsCols; ++j) col[j] = 4U * (unsigned)clampi(X0 - 2 * R + lane + 32 * j, 0, in.w - 1) + cw;
     for (int r = warp; r < SR; r += kGsThreads / 32) {
-        const T* row = px<const T>(in, 0, clampi(Y0 - 2 * R + r, 0, in.h - 1)) + cw;
-        float* dst = sv + r * PV;
-        for (int q = lane; q < SC; q += 32) gs_cp4(dst + q, row + 4 * clampi(X0 - 2 * R + q, 0, in.w - 1));
+        const T* row = px<const T>(in, 0, clampi(Y0 - 2 * R + r, 0, in.h - 1));
+        float* dst = sv + r * PV + lane;
+#pragma unroll
+        for (int j = 0; j < kGsCols; ++j)
+            if (lane + 32 * j < SC) gs_cp4(dst + 32 * j, row + col[j]);
     }
     gs_cp_wait();
     __syncthreads();
-    // row pass: one window per thread, rows on the lanes (SR <= 64 rows)
-    {
-        const int r = threadIdx.x & 63, x0 = (threadIdx.x >> 6) * kGsRunX;
-        if (r < SR) {
+    // row pass: a window per thread, rows on the lanes (SR <= 64 rows, four windows each)
+    if (threadIdx.x < SR * (kGsTW / kGsRunX)) {
+        const int win = threadIdx.x / SR, r = threadIdx.x - win * SR, x0 = win * kGsRunX;
         const uint32_t* row = reinterpret_cast<const uint32_t*>(sv) + r * PV + x0;
-        float2 s = make_float2(0.0F, 0.0F);
-#pragma unroll 4
-        for (int k = 0; k < D; ++k) {
-            const float v = gs_val<T>(row[k], c);
-            s = __fadd2_rn(s, make_float2(v, v * v));
-        }
         float2* o = hs + r * kGsPH + x0;
-        o[0] = s;
-#pragma unroll
-        for (int x = 1; x < kGsRunX; ++x) {
-            const float vi = gs_val<T>(row[x + D - 1], c), vo = gs_val<T>(row[x - 1], c);
-            s = __fadd2_rn(__fadd2_rn(s, make_float2(vi, vi * vi)), make_float2(-vo, -(vo * vo)));
-            o[x] = s;
-        }
-        }
+        gs_slide<kGsRunX, kGsRunX - 1>(
+            D,
+            [&](int k) {
+                const float v = gs_val<T>(row[k], c);
+                return make_float2(v, v * v);
+            },
+            [&](int i, float2 s) { o[i] = s; });
     }
     __syncthreads();
     const float invN = 1.0F / (float)(D * D);
     const int x = threadIdx.x % kGsTW, y0 = (threadIdx.x / kGsTW) * kGsRunY;
     const int xa = X0 + x;
-    float2 S = make_float2(0.0F, 0.0F);
-#pragma unroll 4
-    for (int k = 0; k < D; ++k) S = __fadd2_rn(S, hs[(y0 + k) * kGsPH + x]);
     const size_t plane = (size_t)p.Ha * p.Wa;
     // plane offsets fit 32 bits (Ha * Wa < 2^31 is checked on the host)
     float* pa = p.a + (size_t)c * plane + (unsigned)((Y0 + y0) * p.Wa + xa);
     float* pb = p.b + (size_t)c * plane + (unsigned)((Y0 + y0) * p.Wa + xa);
-    const float2* hin = hs + (y0 + D) * kGsPH + x;
-    const float2* hout = hs + y0 * kGsPH + x;
+    const float2* hcol = hs + y0 * kGsPH + x;
     const int nrow = min(kGsRunY, p.Ha - (Y0 + y0));
-    const bool col = xa < p.Wa;
-#pragma unroll
-    for (int y = 0; y < kGsRunY; ++y) {
-        if (y > 0) S = __fadd2_rn(__fadd2_rn(S, hin[(y - 1) * kGsPH]), neg2(hout[(y - 1) * kGsPH]));
-        if (col && y < nrow) {
+    const bool inside = xa < p.Wa;
+    gs_slide<kGsRunY, kGsRunY - 1>(
+        D, [&](int k) { return hcol[k * kGsPH]; },
+        [&](int y, float2 S) {
+            if (!inside || y >= nrow) return;
             const float2 mc = __fmul2_rn(S, make_float2(invN, invN));  // (m, corr)
             const float var = maxf(mc.y - mc.x * mc.x, 0.0F);
             const float a = __fdividef(var, var + eps);
             pa[y * p.Wa] = a;
             pb[y * p.Wa] = mc.x - a * mc.x;
-        }
-    }
+        });
 }
 
 template <class T>
@@ -200,6 +220,9 @@ __global__ void __launch_bounds__(kGsThreads, 4) gsp_out_kernel(Img in, Img out,
     const int x = threadIdx.x % kGsTW, y0 = (threadIdx.x / kGsTW) * kGsRunY;
     const int gx = X0 + x;
     // output x reads plane columns x .. x + 2R (extended x - R .. x + R)
+    unsigned col[kGsCols];  // the lane's columns, the same in every row
+#pragma unroll
+    for (int j = 0; j < kGsCols; ++j) col[j] = (unsigned)min(X0 + lane + 32 * j, p.Wa - 1);
     auto stage = [&](int c) {
         const float* ca = p.a + (size_t)c * plane;
         const float* cb = p.b + (size_t)c * plane;
@@ -207,12 +230,13 @@ __global__ void __launch_bounds__(kGsThreads, 4) gsp_out_kernel(Img in, Img out,
             const unsigned ro = (unsigned)min(Y0 + r, p.Ha - 1) * (unsigned)p.Wa;
             const float* ra = ca + ro;
             const float* rb = cb + ro;
-            float2* dst = sab + r * PV;
-            for (int q = lane; q < SC; q += 32) {
-                const int xq = min(X0 + q, p.Wa - 1);
-                gs_cp4(&dst[q].x, ra + xq);
-                gs_cp4(&dst[q].y, rb + xq);
-            }
+            float2* dst = sab + r * PV + lane;
+#pragma unroll
+            for (int j = 0; j < kGsCols; ++j)
+                if (lane + 32 * j < SC) {
+                    gs_cp4(&dst[32 * j].x, ra + col[j]);
+                    gs_cp4(&dst[32 * j].y, rb + col[j]);
+                }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
@@ -227,39 +251,24 @@ __global__ void __launch_bounds__(kGsThreads, 4) gsp_out_kernel(Img in, Img out,
     float res[3][kGsRunY];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        if (c > 0) stage(c);  // the previous channel's passes are done with sab
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
-        {
-            const int r = threadIdx.x & 63, x0 = (threadIdx.x >> 6) * kGsRunX;
-            if (r < SR) {
+        if (threadIdx.x < SR * (kGsTW / kGsRunX)) {
+            const int win = threadIdx.x / SR, r = threadIdx.x - win * SR, x0 = win * kGsRunX;
             const float2* row = sab + r * PV + x0;
-            float2 s = make_float2(0.0F, 0.0F);
-#pragma unroll 4
-            for (int k = 0; k < D; ++k) s = __fadd2_rn(s, row[k]);
             float2* o = hs + r * kGsPH + x0;
-            o[0] = s;
-#pragma unroll
-            for (int xx = 1; xx < kGsRunX; ++xx) {
-                s = __fadd2_rn(__fadd2_rn(s, row[xx + D - 1]), neg2(row[xx - 1]));
-                o[xx] = s;
-            }
-            }
+            gs_slide<kGsRunX, kGsKeepOut>(D, [&](int k) { return row[k]; }, [&](int i, float2 s) { o[i] = s; });
         }
         __syncthreads();
-        float2 S = make_float2(0.0F, 0.0F);
-#pragma unroll 4
-        for (int k = 0; k < D; ++k) S = __fadd2_rn(S, hs[(y0 + k) * kGsPH + x]);
-        const float2* hin = hs + (y0 + D) * kGsPH + x;
-        const float2* hout = hs + y0 * kGsPH + x;
-#pragma unroll
-        for (int y = 0; y < kGsRunY; ++y) {
-            if (y > 0) S = __fadd2_rn(__fadd2_rn(S, hin[(y - 1) * kGsPH]), neg2(hout[(y - 1) * kGsPH]));
-            const float2 mab = __fmul2_rn(S, make_float2(invN, invN));  // (mean_a, mean_b)
-            const float v = c == 0 ? vin[y].r : (c == 1 ? vin[y].g : vin[y].b);
-            res[c][y] = max0(mab.x * v + mab.y);
-        }
-        __syncthreads();  // the next channel restages sab and rewrites hs
+        if (c < 2) stage(c + 1);  // sab is free: the next channel comes in under the column pass
+        const float2* hcol = hs + y0 * kGsPH + x;
+        gs_slide<kGsRunY, kGsRunY - 1>(
+            D, [&](int k) { return hcol[k * kGsPH]; },
+            [&](int y, float2 S) {
+                const float2 mab = __fmul2_rn(S, make_float2(invN, invN));  // (mean_a, mean_b)
+                const float v = c == 0 ? vin[y].r : (c == 1 ? vin[y].g : vin[y].b);
+                res[c][y] = max0(mab.x * v + mab.y);
+            });
     }
     if (gx >= p.w) return;
 #pragma unroll
