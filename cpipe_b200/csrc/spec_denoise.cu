@@ -368,14 +368,17 @@ __device__ __forceinline__ void atrous_tap(const Img& in, const float* __restric
 // c_j value is read about once (plus the 4s/(256 - 4s) column halo and the four
 // warm-up rows per walk).  Per output: the vertical B3 taps first, then the
 // horizontal ones, each b3(t[-2s], t[-s], t[0], t[s], t[2s]); the first level
-// (s = 1) reads c_0 = (Y, Co, Cg) from the input frame.
+// (s = 1) reads c_0 = (Y, Co, Cg) from the input frame.  Bound by issue: two
+// buffers for one barrier a step, five steps unrolled so that the taps stay
+// where they are.  12 MP: 70.6 -> 65.7 us (first level, binary16), 71.9 -> 69.8
+// (third), at 40 registers; 48 and 32 registers took 75 and 79.
 constexpr int kAtSeg = 32;  // steps per walk
 __host__ __device__ constexpr int atrous_walk_cols(int s) { return kAtThreads - 4 * s; }
 template <class T, bool FIRST>
-__global__ void __launch_bounds__(kAtThreads) atrous_walk_kernel(Img in, const float* __restrict__ cin,
+__global__ void __launch_bounds__(kAtThreads, 6) atrous_walk_kernel(Img in, const float* __restrict__ cin,
                                                                  float* __restrict__ cout, float* __restrict__ part,
                                                                  int w, int h, long long npx, int s) {
-    __shared__ float vrow[3][kAtThreads];
+    __shared__ float vrow[2][3][kAtThreads];  // a step's vertical results, this step's and the last one's
     const int t = threadIdx.x, OW = atrous_walk_cols(s);
     const int x0 = blockIdx.x * OW;                      // first output column
     const int xc = clampi(x0 - 2 * s + t, 0, w - 1);      // this thread's (clamped) column
@@ -386,36 +389,39 @@ __global__ void __launch_bounds__(kAtThreads) atrous_walk_kernel(Img in, const f
     if (nk > 0) {
         const int x = x0 + t - 2 * s;
         const bool out = t >= 2 * s && t < 2 * s + OW && x < w;
-        float ring[5][3];  // c_j at rows y - 2s .. y + 2s (clamped) of this column
+        float ring[5][3];  // c_j at rows y - 2s .. y + 2s (clamped) of this column, row y + (m - 2) s at (k + m) % 5
         const int yb = phi + s * k0;
 #pragma unroll
         for (int m = 0; m < 5; ++m) atrous_tap<T, FIRST>(in, cin, npx, w, xc, clampi(yb + (m - 2) * s, 0, h - 1), ring[m]);
-        for (int k = 0; k < nk; ++k) {
-            const int y = yb + s * k;
+        for (int kb = 0; kb < nk; kb += 5) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) vrow[c][t] = b3(ring[0][c], ring[1][c], ring[2][c], ring[3][c], ring[4][c]);
-            // the next step's new row, in flight across this step's barriers
-            // (raw words; converted after them)
-            AtrousRaw<T, FIRST> nxt;
-            nxt.fetch(in, cin, npx, w, xc, min(y + 3 * s, h - 1));
-            __syncthreads();
-            if (out) {
-                float* dst = cout + (unsigned)(y * w + x);
+            for (int r = 0; r < 5; ++r) {
+                const int k = kb + r, y = yb + s * k;
+                if (k >= nk) break;
+                float(&buf)[3][kAtThreads] = vrow[k & 1];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float* v = vrow[c] + t;
-                    const float hv = b3(v[-2 * s], v[-s], v[0], v[s], v[2 * s]);
-                    const float d = ring[2][c] - hv;
-                    dst[c * npx] = hv;
-                    acc[c] += d * d;
+                for (int c = 0; c < 3; ++c)
+                    buf[c][t] = b3(ring[r][c], ring[(r + 1) % 5][c], ring[(r + 2) % 5][c], ring[(r + 3) % 5][c],
+                                   ring[(r + 4) % 5][c]);
+                // the next step's new row, in flight across this step's barrier
+                // (raw words; converted after it)
+                AtrousRaw<T, FIRST> nxt;
+                nxt.fetch(in, cin, npx, w, xc, min(y + 3 * s, h - 1));
+                // (the other buffer is rewritten after the next step's barrier, past every read of it)
+                __syncthreads();
+                if (out) {
+                    float* dst = cout + (unsigned)(y * w + x);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float* v = buf[c] + t;
+                        const float hv = b3(v[-2 * s], v[-s], v[0], v[s], v[2 * s]);
+                        const float d = ring[(r + 2) % 5][c] - hv;
+                        dst[c * npx] = hv;
+                        acc[c] += d * d;
+                    }
                 }
+                nxt.value(ring[r]);
             }
-            __syncthreads();  // vrow is rewritten by the next step
-#pragma unroll
-            for (int m = 0; m < 4; ++m)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) ring[m][c] = ring[m + 1][c];
-            nxt.value(ring[4]);
         }
     }
     atrous_tile_sums(acc, part);
