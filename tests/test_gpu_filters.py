@@ -89,6 +89,18 @@ def test_qbc_remosaic_filter_bit_exact(cuda_device, h, w):
     np.testing.assert_array_equal(out, oracle.qbc_remosaic(raw))
 
 
+# 64x64 tiles: one whole inside its halo of 3, one column or row short of it, two of them; flat (the largest weights),
+# saturated steps (the smallest)
+@pytest.mark.parametrize("h,w", [(131, 131), (130, 131), (131, 130), (195, 259), (64, 400)])
+@pytest.mark.parametrize("kind", ["noise", "flat", "steps"])
+def test_qbc_remosaic_whole_tiles_bit_exact(cuda_device, h, w, kind):
+    rng = np.random.default_rng(h + w)
+    raw = {"noise": rng.integers(0, 65536, (h, w)), "flat": np.full((h, w), 65535),
+           "steps": 65535 * rng.integers(0, 2, (h, w))}[kind].astype(np.uint16)
+    out = run("demosaic_quad_bayer_remosaic", [raw], [np.zeros_like(raw)])
+    np.testing.assert_array_equal(out, oracle.qbc_remosaic(raw))
+
+
 RGBA_CASES = [
     ("wb_dual_illuminant", lambda: blobs.wb([0.5, 1.0, 0.625]), lambda x, f: oracle.wb(x, [0.5, 1.0, 0.625], f)),
     ("colormatrix_dng_to_working", lambda: blobs.colormatrix([1.7, -0.4, -0.3, -0.2, 1.5, -0.3, 0.05, -0.3, 1.25]),
