@@ -56,6 +56,212 @@ template <int ALGO, class TOut, int TW, int TH>
 __global__ void __launch_bounds__(256) raw_to_rgba_kernel(Img raw, Img out, RawParams p) {
     demosaic_tile<ALGO, TOut, TW, TH>(RawLoader{raw, &p}, raw.w, raw.h, out, p.cfa);
 }
+// Two neighbouring pixels (the second only if `two`).
+__device__ __forceinline__ void store_pair(const Img& out, __half* p, const Rgba& a, const Rgba& b, bool two) {
+    if (two && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && out.pix_stride == 4) {
+        __align__(16) __half2 h[4] = {__floats2half2_rn(a.r, a.g), __floats2half2_rn(a.b, a.a),
+                                      __floats2half2_rn(b.r, b.g), __floats2half2_rn(b.b, b.a)};
+        *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+        return;
+    }
+    store_rgba(p, a);
+    if (two) store_rgba(p + out.pix_stride, b);
+}
+__device__ __forceinline__ void store_pair(const Img& out, float* p, const Rgba& a, const Rgba& b, bool two) {
+    store_rgba(p, a);
+    if (two) store_rgba(p + out.pix_stride, b);
+}
+// RCD and AMaZE of a Bayer mosaic, a warp to a strip of 56 columns, without shared
+// memory.  A lane holds two neighbouring columns, of which one is green in every
+// row, and walks down: at row y it loads row y, finds the green of row y - 2 and
+// writes row y - 3; neighbouring columns come by shuffles, rows from a ring of six
+// in registers (the loop is unrolled by six).  Which column is green is known at
+// compile time, so a site computes what it needs: green and the ratio (RCD) or
+// chroma (AMaZE) at red and blue sites only, a quarter of a full tile's work per
+// site, where demosaic_tile evaluates every site's cases for every pixel.
+// 28 of 32 lanes write; 6 of R + 6 rows are walked twice.  Bound by issue, at 20
+// warps an SM (24 would spill: 99 us).  12 MP, binary16: RCD 124 -> 84 us; 50 MP,
+// AMaZE: 507 -> 280 us; 2015 x 1511 in binary32, RCD: 30 -> 20 us.
+constexpr int kStrip = 56, kStripHalo = 4, kStripWarps = 4;
+struct StripTap {
+    float c, l1, r1, u1, d1, l2, r2, u2, d2;
+    __device__ __forceinline__ float operator()(int dx, int dy) const {
+        return dx == 0 && dy == 0 ? c : dx == -1 ? l1 : dx == 1 ? r1 : dy == -1 ? u1 : dy == 1 ? d1 : dx == -2 ? l2
+               : dx == 2 ? r2 : dy == -2 ? u2 : d2;
+    }
+};
+// A lane's two columns of the raw frame: loads in three steps (gain row samples,
+// raw and gain values, the arithmetic of RawLoader), so that each is in flight
+// while the rows before it are worked on.
+struct StripSource {
+    struct Samples {
+        AxisSample s[2];
+    };
+    struct Words {
+        uint16_t v[2];
+        float lo[2], hi[2], weight[2];
+    };
+    const RawParams& p;
+    const Img& raw;
+    int col[2];
+    float black[2][2], denom[2][2], inv[2][2];
+    bool fast;  // divisions by the denominators' reciprocals (warp-uniform)
+    const float* hrow[2][2];
+    const AxisSample* rows[2][2];
+    __device__ __forceinline__ StripSource(const Img& r, const RawParams& q, int x) : p(q), raw(r) {
+        fast = true;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float d = p.black.denom[i], b = p.black.black[i];
+            fast = fast && d >= 0x1p-10F && d <= 0x1p40F && (__float_as_int(d) & 0x7FFFFF) != 0x7FFFFF && b >= 0.0F && b <= 0x1p20F;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int gx = clampi(x + k, 0, raw.w - 1);
+            col[k] = gx * raw.pix_stride;
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                black[b][k] = p.black.black[2 * b + (gx & 1)];
+                denom[b][k] = p.black.denom[2 * b + (gx & 1)];
+                inv[b][k] = 1.0F / denom[b][k];
+                if (p.has_gain) {
+                    const int m = p.gain.map_count == 1 ? 0 : p.gain.plane_to_map[2 * b + (p.gain.qbc ? (gx % 4) / 2 : gx & 1)];
+                    hrow[b][k] = p.gain.hrow[m] + gx;
+                    rows[b][k] = p.gain.rows[m];
+                }
+            }
+        }
+    }
+    // x / d, correctly rounded, by Markstein's method: the first step brings x inv within an ulp of
+    // the quotient, which the second rounds (inv = RN(1/d), d's significand not all ones; x is 0 or
+    // a difference of sample values, so that nothing underflows)
+    static __device__ __forceinline__ float divide(float x, float d, float inv) {
+        float q = x * inv;
+        q = __fmaf_rn(__fmaf_rn(-q, d, x), inv, q);
+        return __fmaf_rn(__fmaf_rn(-q, d, x), inv, q);
+    }
+    __device__ __forceinline__ int gain_row(int gy) const { return p.gain.qbc ? (gy % 4) / 2 : gy & 1; }
+    __device__ __forceinline__ void samples(int y, Samples& s) const {
+        if (!p.has_gain) return;
+        const int gy = clampi(y, 0, raw.h - 1), b = gain_row(gy);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) s.s[k] = (b ? rows[1][k] : rows[0][k])[gy];
+    }
+    __device__ __forceinline__ void words(int y, const Samples& s, Words& w) const {
+        const int gy = clampi(y, 0, raw.h - 1);
+        const uint16_t* r = px<const uint16_t>(raw, 0, gy);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) w.v[k] = r[col[k]];
+        if (!p.has_gain) return;
+        const int b = gain_row(gy);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float* h = b ? hrow[1][k] : hrow[0][k];
+            w.lo[k] = __ldg(h + (size_t)s.s[k].low * p.gain.hw);
+            w.hi[k] = __ldg(h + (size_t)s.s[k].high * p.gain.hw);
+            w.weight[k] = s.s[k].weight;
+        }
+    }
+    __device__ __forceinline__ void values(int y, const Words& w, float (&v)[2]) const {
+        const int b = clampi(y, 0, raw.h - 1) & 1;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float x = (float)w.v[k] - (b ? black[1][k] : black[0][k]), d = b ? denom[1][k] : denom[0][k];
+            v[k] = clampf(fast ? divide(x, d, b ? inv[1][k] : inv[0][k]) : x / d, 0.0F, 1.0F);
+            if (p.has_gain) v[k] = v[k] * lerpf(w.lo[k], w.hi[k], w.weight[k]);
+        }
+    }
+};
+// E: the column (0 or 1) of the red or blue site of even rows.
+template <int ALGO, class TOut, int E>
+__global__ void __launch_bounds__(32 * kStripWarps) raw_strip_kernel(const __grid_constant__ Img raw, const __grid_constant__ Img out,
+                                                                      const __grid_constant__ RawParams p, int R) {
+    constexpr unsigned kAll = 0xFFFFFFFFU;
+    const int lane = threadIdx.x & 31, ys = (blockIdx.y * kStripWarps + (threadIdx.x >> 5)) * R;
+    const int x = (int)blockIdx.x * kStrip - kStripHalo + 2 * lane;
+    if (ys >= raw.h) return;  // warp-uniform
+    const StripSource src(raw, p, x);
+    const bool red_even = p.cfa.p[E] == 0;  // even rows hold red (else blue)
+    const bool on = lane >= kStripHalo / 2 && lane < 32 - kStripHalo / 2;
+    float V[6][2] = {}, Q[3] = {}, N[3] = {};  // rows by y mod 6 or 3: values; ratio or chroma, and its neighbour's
+    float g_last = 0.0F;                       // green of the last row's red or blue site
+    StripSource::Samples s1, s2;
+    StripSource::Words w0, w1;
+    src.samples(ys - 3, s1);
+    src.samples(ys - 2, s2);
+    src.words(ys - 3, s1, w0);
+    for (int t = 0; t < R + 6; t += 6) {
+        if (ys + t - 6 >= raw.h) break;  // warp-uniform
+#pragma unroll
+        for (int s = 0; s < 6; ++s) {
+            const int y = ys - 3 + t + s;           // ys is even: row y is odd for even s
+            constexpr int kOdd[6] = {1, 0, 1, 0, 1, 0};
+            const int n = kOdd[s] ? 1 - E : E;      // the red or blue column of rows y, y - 2
+            src.samples(y + 2, s1);
+            src.words(y + 1, s2, w1);
+            src.values(y, w0, V[s]);
+            // green of row y - 2's red or blue site
+            const float(&c)[2] = V[(s + 4) % 6];
+            const float other = n == 0 ? __shfl_up_sync(kAll, c[1], 1) : __shfl_down_sync(kAll, c[0], 1);
+            const float left = __shfl_up_sync(kAll, c[n], 1), right = __shfl_down_sync(kAll, c[n], 1);
+            const StripTap T{c[n], n == 0 ? other : c[0], n == 0 ? c[1] : other, V[(s + 3) % 6][n], V[(s + 5) % 6][n],
+                             left, right, V[(s + 2) % 6][n], V[s][n]};
+            const float g = ALGO == 1 ? rcd_green(T) : amaze_green(T);
+            const float q = ALGO == 1 ? c[n] / maxf(g, 0.000001F) : c[n] - g;
+            constexpr int kM = 3;
+            Q[(s + 4) % kM] = q;
+            N[(s + 4) % kM] = n == 0 ? __shfl_down_sync(kAll, q, 1) : __shfl_up_sync(kAll, q, 1);
+            // row y - 3: its red or blue column is m, the rows beside it have theirs in the other
+            if (t > 0) {
+                const int m = 1 - n, yo = y - 3;
+                const float(&o)[2] = V[(s + 3) % 6];
+                const float qu = Q[(s + 2) % kM], qd = Q[(s + 4) % kM], nu = N[(s + 2) % kM], nd = N[(s + 4) % kM];
+                const float q0 = Q[s % kM], n0 = N[s % kM];
+                // left to right: the neighbour's column, then the lane's own, or the other way round
+                const float diag = m == 0 ? nu + qu + nd + qd : qu + nu + qd + nd;
+                const float hor = m == 0 ? q0 + n0 : n0 + q0, ver = qu + qd, gc = o[1 - m];
+                float vo, gh, gv;  // the other colour at the red or blue site; both at the green one
+                if (ALGO == 1) {
+                    vo = g_last * 0.25F * diag;
+                    gh = gc * 0.5F * hor;
+                    gv = gc * 0.5F * ver;
+                } else {
+                    vo = g_last + 0.25F * diag;
+                    gh = gc + 0.5F * hor;
+                    gv = gc + 0.5F * ver;
+                }
+                const bool red = kOdd[s] ? red_even : !red_even;  // row y - 3 has the other parity than row y
+                const float site_c = max0(o[m]), site_o = max0(vo), gr_c = max0(gh), gr_o = max0(gv);
+                Rgba px2[2];
+                px2[m] = Rgba{red ? site_c : site_o, max0(g_last), red ? site_o : site_c, 1.0F};
+                px2[1 - m] = Rgba{red ? gr_c : gr_o, max0(gc), red ? gr_o : gr_c, 1.0F};
+                if (on && yo < out.h && x < out.w) {
+                    TOut* d = px<TOut>(out, x, yo);
+                    store_pair(out, d, px2[0], px2[1], x + 1 < out.w);
+                }
+            }
+            g_last = g;
+            s2 = s1;
+            w0 = w1;
+        }
+    }
+}
+template <int ALGO, class TOut>
+bool launch_raw_strips(const Img& raw, const Img& out, const RawParams& p, cudaStream_t st) {
+    const int* c = p.cfa.p;
+    const auto pair = [](int a, int b) { return (a == 0 && b == 2) || (a == 2 && b == 0); };
+    const int e = c[1] == 1 && c[2] == 1 && pair(c[0], c[3]) ? 0 : c[0] == 1 && c[3] == 1 && pair(c[1], c[2]) ? 1 : -1;
+    if (e < 0 || raw.w != out.w || raw.h != out.h) return false;
+    // rows a warp: the six rows walked twice cost less the more there are, while there are warps
+    // enough for the chip (50 MP, AMaZE: 36 rows 280 us, 24 rows 299, 12 rows 359; 12 MP, RCD: 84, 84, 95)
+    const unsigned cols = (unsigned)((raw.w + kStrip - 1) / kStrip);
+    auto warps = [&](int R) { return (long long)cols * ((raw.h + R - 1) / R); };
+    const int R = warps(36) >= kSmCount * 64 ? 36 : warps(24) >= kSmCount * 12 ? 24 : 12;
+    const dim3 g(cols, (unsigned)((raw.h + R * kStripWarps - 1) / (R * kStripWarps)));
+    if (e == 0) raw_strip_kernel<ALGO, TOut, 0><<<g, 32 * kStripWarps, 0, st>>>(raw, out, p, R);
+    else raw_strip_kernel<ALGO, TOut, 1><<<g, 32 * kStripWarps, 0, st>>>(raw, out, p, R);
+    return true;
+}
 template <int ALGO, class TOut>
 void launch_raw_to_rgba(const Img& raw, const Img& out, const RawParams& p, cudaStream_t st) {
     const dim3 g((unsigned)((raw.w + kDmTW - 1) / kDmTW), (unsigned)((raw.h + kDmTH - 1) / kDmTH));
@@ -63,6 +269,12 @@ void launch_raw_to_rgba(const Img& raw, const Img& out, const RawParams& p, cuda
         const dim3 gs((unsigned)((raw.w + kDmTWs - 1) / kDmTWs), (unsigned)((raw.h + kDmTHs - 1) / kDmTHs));
         raw_to_rgba_kernel<ALGO, TOut, kDmTWs, kDmTHs><<<gs, kDmThreads, 0, st>>>(raw, out, p);
     } else {
+        // Strips from about 1 MP on: with fewer tiles than 6 to an SM a warp's dependent rows take
+        // longer than the tiles (two kernels of the chain, 640 x 480: 18.3 against 16.5 us; 1008 x 756:
+        // 28.7 and 28.7; 2048 x 1536: 84 and 94).
+        if constexpr (ALGO != 0) {
+            if ((long long)g.x * g.y >= 6 * kSmCount && launch_raw_strips<ALGO, TOut>(raw, out, p, st)) return;
+        }
         raw_to_rgba_kernel<ALGO, TOut, kDmTW, kDmTH><<<g, kDmThreads, 0, st>>>(raw, out, p);
     }
 }
@@ -225,20 +437,6 @@ __device__ __forceinline__ void load_block(const Img& in, int u, int v, Rgba (&q
         q[2] = load_rgba(px<const T>(in, u, v1));
         q[3] = load_rgba(px<const T>(in, u1, v1));
     }
-}
-__device__ __forceinline__ void store_pair(const Img& out, __half* p, const Rgba& a, const Rgba& b, bool two) {
-    if (two && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && out.pix_stride == 4) {
-        __align__(16) __half2 h[4] = {__floats2half2_rn(a.r, a.g), __floats2half2_rn(a.b, a.a),
-                                      __floats2half2_rn(b.r, b.g), __floats2half2_rn(b.b, b.a)};
-        *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
-        return;
-    }
-    store_rgba(p, a);
-    if (two) store_rgba(p + out.pix_stride, b);
-}
-__device__ __forceinline__ void store_pair(const Img& out, float* p, const Rgba& a, const Rgba& b, bool two) {
-    store_rgba(p, a);
-    if (two) store_rgba(p + out.pix_stride, b);
 }
 // Wavelet, tone and LUT on the aligned 2x2 block at (x, y): q its (guided)
 // values, alpha included; cells outside the frame hold their clamped neighbour.

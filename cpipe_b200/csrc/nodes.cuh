@@ -73,24 +73,25 @@ struct Cfa {
     __device__ __forceinline__ int at(int x, int y) const { return p[((y & 1) * 2) + (x & 1)]; }
 };
 
-// demosaic_rcd_generator.cpp:28-35
+// demosaic_rcd_generator.cpp:28-35, at a red or blue site
 template <class Tap>
-__device__ __forceinline__ float rcd_green(const Tap& T, int x, int y, const Cfa& cfa) {
-    const float c = T(0, 0);
+__device__ __forceinline__ float rcd_green(const Tap& T) {
     const float gh = 0.5F * (T(-1, 0) + T(1, 0));
     const float gv = 0.5F * (T(0, -1) + T(0, 1));
     const float dh = fabsf(T(-2, 0) - T(2, 0));
     const float dv = fabsf(T(0, -2) - T(0, 2));
-    if (cfa.at(x, y) == 1) return c;
     if (dh < dv) return gh;
     if (dv < dh) return gv;
     return 0.5F * (gh + gv);
 }
-// demosaic_amaze_generator.cpp:24-46
 template <class Tap>
-__device__ __forceinline__ float amaze_green(const Tap& T, int x, int y, const Cfa& cfa) {
+__device__ __forceinline__ float rcd_green(const Tap& T, int x, int y, const Cfa& cfa) {
+    return cfa.at(x, y) == 1 ? T(0, 0) : rcd_green(T);
+}
+// demosaic_amaze_generator.cpp:24-46, at a red or blue site
+template <class Tap>
+__device__ __forceinline__ float amaze_green(const Tap& T) {
     const float c = T(0, 0);
-    if (cfa.at(x, y) == 1) return c;
     const float ct = 2.0F * c;
     const float ghn = T(-1, 0) + T(1, 0);
     const float gvn = T(0, -1) + T(0, 1);
@@ -103,6 +104,10 @@ __device__ __forceinline__ float amaze_green(const Tap& T, int x, int y, const C
     if (grh < grv) return gh;
     if (grv < grh) return gv;
     return 0.5F * (gh + gv);
+}
+template <class Tap>
+__device__ __forceinline__ float amaze_green(const Tap& T, int x, int y, const Cfa& cfa) {
+    return cfa.at(x, y) == 1 ? T(0, 0) : amaze_green(T);
 }
 
 // ------------------------------------------------------------ RGBA pixel ops

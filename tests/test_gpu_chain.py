@@ -155,6 +155,22 @@ def test_chain_tile_sizes_equal_nodes(cuda_device, host, w, h, radius):
     chain.close()
 
 
+# from 6 tiles an SM on a Bayer demosaic walks strips of 56 columns: the last strip cut to 55, 56, 1 and 2 columns, last
+# rows of a walk of 12 and 24 cut, each place of green, both colours first; denominators whose reciprocal is and is not
+# used (all ones: 512 - 2^-15)
+@pytest.mark.parametrize("w,h,variant", [
+    (1007, 911, dict()), (1008, 912, dict(cfa=(1, 0, 2, 1), gainmap=False)), (1009, 910, dict(cfa=(1, 2, 0, 1), black=16.3)),
+    (1010, 913, dict(cfa=(2, 1, 1, 0), demosaic="amaze", black=511.000030517578125)), (2015, 1511, dict(demosaic="amaze")),
+    (57, 14200, dict(demosaic="amaze", gainmap=False))])
+def test_chain_strip_demosaic_equals_nodes(cuda_device, host, w, h, variant):
+    cfg = ChainConfig.small(w, h, guided_radius=0, **variant)
+    raw = np.random.default_rng(w + h).integers(0, 1024, (h, w)).astype(np.uint16)
+    chain = Chain(cfg)
+    fused = chain.run_host(raw)
+    assert f16_ulp_distance(fused, run_nodes_on_gpu(host, cfg, raw)).max() == 0
+    chain.close()
+
+
 def test_chain_general_opcode_list(cuda_device):
     """OpcodeList3 lists other than a single warp take the per-node path inside the chain."""
     import ctypes as C
