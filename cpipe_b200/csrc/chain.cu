@@ -172,14 +172,12 @@ struct StripSource {
         }
     }
 };
-// E: the column (0 or 1) of the red or blue site of even rows.
+// Rows ys .. ys + R - 1 (ys even, R a multiple of 6) of the strip of columns xs .. xs + 55.  E: the column
+// (0 or 1) of the red or blue site of even rows.
 template <int ALGO, class TOut, int E>
-__global__ void __launch_bounds__(32 * kStripWarps) raw_strip_kernel(const __grid_constant__ Img raw, const __grid_constant__ Img out,
-                                                                      const __grid_constant__ RawParams p, int R) {
+__device__ __forceinline__ void strip_walk(const Img& raw, const Img& out, const RawParams& p, int xs, int ys, int R) {
     constexpr unsigned kAll = 0xFFFFFFFFU;
-    const int lane = threadIdx.x & 31, ys = (blockIdx.y * kStripWarps + (threadIdx.x >> 5)) * R;
-    const int x = (int)blockIdx.x * kStrip - kStripHalo + 2 * lane;
-    if (ys >= raw.h) return;  // warp-uniform
+    const int lane = threadIdx.x & 31, x = xs - kStripHalo + 2 * lane;
     const StripSource src(raw, p, x);
     const bool red_even = p.cfa.p[E] == 0;  // even rows hold red (else blue)
     const bool on = lane >= kStripHalo / 2 && lane < 32 - kStripHalo / 2;
@@ -246,11 +244,21 @@ __global__ void __launch_bounds__(32 * kStripWarps) raw_strip_kernel(const __gri
         }
     }
 }
+template <int ALGO, class TOut, int E>
+__global__ void __launch_bounds__(32 * kStripWarps) raw_strip_kernel(const __grid_constant__ Img raw, const __grid_constant__ Img out,
+                                                                      const __grid_constant__ RawParams p, int R) {
+    const int ys = (blockIdx.y * kStripWarps + (threadIdx.x >> 5)) * R;
+    if (ys < raw.h) strip_walk<ALGO, TOut, E>(raw, out, p, (int)blockIdx.x * kStrip, ys, R);
+}
+// Column of the red or blue site of even rows of a Bayer mosaic, -1 for any other.
+int strip_phase(const Cfa& cfa) {
+    const int* c = cfa.p;
+    const auto pair = [](int a, int b) { return (a == 0 && b == 2) || (a == 2 && b == 0); };
+    return c[1] == 1 && c[2] == 1 && pair(c[0], c[3]) ? 0 : c[0] == 1 && c[3] == 1 && pair(c[1], c[2]) ? 1 : -1;
+}
 template <int ALGO, class TOut>
 bool launch_raw_strips(const Img& raw, const Img& out, const RawParams& p, cudaStream_t st) {
-    const int* c = p.cfa.p;
-    const auto pair = [](int a, int b) { return (a == 0 && b == 2) || (a == 2 && b == 0); };
-    const int e = c[1] == 1 && c[2] == 1 && pair(c[0], c[3]) ? 0 : c[0] == 1 && c[3] == 1 && pair(c[1], c[2]) ? 1 : -1;
+    const int e = strip_phase(p.cfa);
     if (e < 0 || raw.w != out.w || raw.h != out.h) return false;
     // rows a warp: the six rows walked twice cost less the more there are, while there are warps
     // enough for the chip (50 MP, AMaZE: 36 rows 280 us, 24 rows 299, 12 rows 359; 12 MP, RCD: 84, 84, 95)
@@ -1505,6 +1513,7 @@ struct Frame {
     ColorParams color;
     ToneParams tone;
     int t1x, t2x, t3x;  // work items per row, per stage
+    int strip;          // stage 1 by strips: strip_phase of the mosaic, -1 by tiles
     int rows2;          // rows per stage-2 work item (autotuned)
 };
 
@@ -1548,8 +1557,12 @@ __device__ __forceinline__ int next_item(const Frame* __restrict__ frames, const
     return t - s_prefix[f];
 }
 
+// (A strip item is eight walks of kItemRows rows, one above the other.  Eight frames of 1 to 6 MP: 2295
+// -> 2225 us a batch against tiles; two CTAs an SM at 128 registers, with a few spilled, as the frame's
+// parameters come from shared memory.)
+constexpr int kItemRows = 24;
 template <int ALGO>
-__global__ void __launch_bounds__(256) batch_raw_kernel(const Frame* __restrict__ frames,
+__global__ void __launch_bounds__(256, 2) batch_raw_kernel(const Frame* __restrict__ frames,
                                                         const int* __restrict__ prefix, int n) {
     __shared__ int s_prefix[kMaxFrames + 1];
     __shared__ Frame s_f;
@@ -1558,8 +1571,20 @@ __global__ void __launch_bounds__(256) batch_raw_kernel(const Frame* __restrict_
     int cur = -1;
     for (int t = blockIdx.x; t < s_prefix[n]; t += gridDim.x) {
         const int local = next_item(frames, s_prefix, n, t, &s_f, &cur);
+        const int tx = local % s_f.t1x, ty = local / s_f.t1x;
+        if constexpr (ALGO != 0) {
+            if (s_f.strip >= 0) {
+                const int ys = (8 * ty + (int)(threadIdx.x >> 5)) * kItemRows;
+                if (ys < s_f.bayer.h) {
+                    if (s_f.strip == 0) strip_walk<ALGO, __half, 0>(s_f.bayer, s_f.mid0, s_f.raw, tx * kStrip, ys, kItemRows);
+                    else strip_walk<ALGO, __half, 1>(s_f.bayer, s_f.mid0, s_f.raw, tx * kStrip, ys, kItemRows);
+                }
+                __syncthreads();
+                continue;
+            }
+        }
         demosaic_tile_at<ALGO, __half>(RawLoader{s_f.bayer, &s_f.raw}, s_f.bayer.w, s_f.bayer.h, s_f.mid0, s_f.raw.cfa,
-                                       (local % s_f.t1x) * kDmTW, (local / s_f.t1x) * kDmTH);
+                                       tx * kDmTW, ty * kDmTH);
         __syncthreads();
     }
 }
@@ -1700,7 +1725,8 @@ int batch_prefix(cpipe_cuda_batch* b) {
         cpb::batch::Frame& f = b->frames[i];
         const int h = f.mid0.h;
         f.rows2 = b->rows2;
-        b->prefix[0 * (n + 1) + i + 1] = b->prefix[0 * (n + 1) + i] + f.t1x * ((h + kDmTH - 1) / kDmTH);
+        b->prefix[0 * (n + 1) + i + 1] = b->prefix[0 * (n + 1) + i] + f.t1x * ((h + (f.strip >= 0 ? 8 * cpb::batch::kItemRows : kDmTH) - 1) /
+                                                                                (f.strip >= 0 ? 8 * cpb::batch::kItemRows : kDmTH));
         b->prefix[1 * (n + 1) + i + 1] = b->prefix[1 * (n + 1) + i] + f.t2x * ((h + b->rows2 - 1) / b->rows2);
         b->prefix[2 * (n + 1) + i + 1] = b->prefix[2 * (n + 1) + i] + f.t3x * ((h + kCTH - 1) / kCTH);
     }
@@ -1776,6 +1802,7 @@ cpipe_cuda_batch* cpipe_cuda_batch_create(const cpipe_cuda_chain_config* cfgs, s
         shared.sg = b->shared_sg;
         shared.d_denoise = b->shared_denoise;
     }
+    long long tiles = 0;  // of 64 x 16, over all frames
     for (size_t i = 0; i < n; ++i) {
         cpipe_cuda_chain_config c = cfgs[i];
         if (c.plain_f32 || c.denoise_mode != b->denoise_mode || c.stop_after != 0 || c.guided_spec || c.atrous_levels ||
@@ -1808,11 +1835,19 @@ cpipe_cuda_batch* cpipe_cuda_batch_create(const cpipe_cuda_chain_config* cfgs, s
         f.taps = WarpTaps{ch->d_taps_ixy, ch->d_taps_tx, ch->d_taps_ty};
         f.color = ch->color;
         f.tone = ch->tone;
+        f.strip = -1;
         f.t1x = (w + kDmTW - 1) / kDmTW;
+        tiles += (long long)f.t1x * ((h + kDmTH - 1) / kDmTH);
         f.t2x = (w + 127) / 128;
         f.t3x = (w + kCTW - 1) / kCTW;
         b->frames.push_back(f);
     }
+    // Bayer frames by strips where the batch makes some items for every SM (two from 3.6 MP on)
+    if (b->algo != 0 && tiles >= 24LL * kSmCount)
+        for (Frame& f : b->frames) {
+            f.strip = cpb::strip_phase(f.raw.cfa);
+            if (f.strip >= 0) f.t1x = (f.mid0.w + kStrip - 1) / kStrip;
+        }
     if (cudaMalloc(&b->d_frames, sizeof(Frame) * n) != cudaSuccess ||
         cudaMalloc(&b->d_prefix, sizeof(int) * 3 * (n + 1)) != cudaSuccess ||
         cudaMalloc(&b->d_left, sizeof(int) * n) != cudaSuccess ||

@@ -159,3 +159,26 @@ def test_batch_frame_times_cover_the_run(cuda_device):
     batch.close()
     for p in d_raw + d_out:
         A.lib().cpipe_cuda_device_free(C.c_void_p(p))
+
+
+@pytest.mark.parametrize("demosaic", ["rcd", "amaze"])
+def test_batch_by_strips_equals_single_frame_chains(cuda_device, demosaic):
+    """From 3.6 MP in all the first stage walks strips; the small frames' own chains use tiles."""
+    frames = B.workload(7, seed=41, mp_range=(0.2, 1.6), demosaic=demosaic)
+    assert sum(c.width * c.height for c, _ in frames) > 3.7e6 and len({k for _, k in frames}) > 1
+    d_raw = [alloc(c.width * c.height * 2) for c, _ in frames]
+    d_out = [alloc(c.width * c.height * 8) for c, _ in frames]
+    for p, (c, k) in zip(d_raw, frames):
+        B.scene_raw(p, c, k)
+    batch = B.Batch([c for c, _ in frames])
+    batch.run(d_raw, d_out)
+    got = [download(p, (c.height, c.width, 4), np.float16) for p, (c, _) in zip(d_out, frames)]
+    for i, (c, k) in enumerate(frames):
+        ch = Chain(c)
+        ch.run(d_raw[i], d_out[i])
+        want = download(d_out[i], (c.height, c.width, 4), np.float16)
+        np.testing.assert_array_equal(got[i].view(np.uint16), want.view(np.uint16), err_msg=f"{k} {c.name}")
+        ch.close()
+    batch.close()
+    for p in d_raw + d_out:
+        A.lib().cpipe_cuda_device_free(C.c_void_p(p))
