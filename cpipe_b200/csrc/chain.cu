@@ -670,7 +670,8 @@ __global__ void gather_kernel(Img src, T* __restrict__ dst, int edge, SpotOrigin
 // Mean squared RGB difference between the frame (at the origins) and the
 // reference tiles, in two steps: mse_kernel sums kMseRows rows of one tile per
 // CTA into part[tile][chunk]; decide_kernel adds a tile's chunks in a fixed
-// order (so the decision does not depend on scheduling) and tests the worst tile.
+// order (so the decision does not depend on scheduling) and tests each tile: one
+// over the limit, or whose error is not finite (counted as infinite), falls back.
 constexpr int kMseRows = 8;
 constexpr int kMseChunks = 256 / kMseRows;  // chunks per tile at the largest edge (256)
 template <class T>
@@ -700,15 +701,18 @@ __global__ void decide_kernel(const float* __restrict__ part, int n, int edge, f
                               SpotStats* stats) {
     const int chunks = (edge + kMseRows - 1) / kMseRows;
     float worst = 0.0F;
+    bool over = false;
     if ((int)threadIdx.x < n) {  // a lane per tile (one thread for all of them took 13 us)
         float s = 0.0F;
         for (int k = 0; k < chunks; ++k) s += part[threadIdx.x * kMseChunks + k];
-        worst = fmaxf(worst, s / (3.0F * (float)(edge * edge)));
+        const float mse = s / (3.0F * (float)(edge * edge));
+        over = !(mse <= mse_max);  // (true for a NaN, which fmaxf below would drop)
+        worst = mse >= 0.0F ? mse : INFINITY;
     }
+    const int fall = __any_sync(0xFFFFFFFFU, over);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xFFFFFFFFU, worst, off));
     if (threadIdx.x != 0) return;
-    const int fall = !(worst <= mse_max);  // a non-finite tile error also falls back
     *gate = fall;
     stats->frames += 1U;
     stats->fallbacks += (unsigned)fall;

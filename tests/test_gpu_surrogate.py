@@ -205,6 +205,30 @@ def test_spot_check_falls_back_to_bm3d(cuda_device):
     bm3d.close()
 
 
+def test_spot_check_falls_back_on_a_nan(cuda_device):
+    """A network whose output is NaN (the last layer sums Inf - Inf) fails its spot check, also at a
+    threshold that any number passes; the frame is then BM3D's."""
+    params = S.init_params(6)
+    for l in (5, 6, 7):
+        params[l][0][:] = 0.0
+    params[5][1][0] = 3e38
+    params[6][0][:2, 0, 1, 1] = 3e38  # two channels of Inf
+    params[7][0][:, 0, 1, 1], params[7][0][:, 1, 1, 1] = 1.0, -1.0
+    blob = S.to_blob(params)
+    raw = ChainConfig.full_12mp(width=320, height=288).make_raw()
+    plain = Chain(ChainConfig.full_12mp(width=320, height=288, surrogate_blob=blob, denoise="surrogate",
+                                        spot_tiles=0, stop_after=2))
+    assert np.isnan(plain.run_host(raw)[8:-8, :, :3].astype(np.float32)).all()
+    checked = spot_chain(blob, 0.0, stop_after=2)
+    got = checked.run_host(raw).astype(np.float32)
+    assert checked.denoise_stats() == (1, 1, float("-inf"))
+    bm3d = Chain(ChainConfig.full_12mp(width=320, height=288, denoise="bm3d", stop_after=2))
+    want = bm3d.run_host(raw).astype(np.float32)
+    assert 10 * np.log10(1.0 / np.mean((got[..., :3] - want[..., :3]) ** 2)) >= 60.0
+    for c in (plain, checked, bm3d):
+        c.close()
+
+
 @pytest.mark.skipif(not os.path.exists(S.DEFAULT_WEIGHTS), reason="no trained weights committed")
 def test_trained_surrogate_passes_spot_check_at_12mp(cuda_device):
     """The committed network on the 4032x3024 benchmark frame: every sampled
