@@ -1277,27 +1277,22 @@ int bm3d_plan(const cpipe_Bm3dSpecParams* p, int w, int h, Bm3dPlan* out, int ba
 
 cudaError_t bm3d_setup(const Bm3dPlan& p) {
     if (p.copy) return cudaSuccess;
-    static const size_t kSmemOptIn = 227 * 1024;
-    const size_t ms = p.match_bytes, fs1 = filter_smem(p, 1), fs2 = filter_smem(p, 2);
-    if (ms > kSmemOptIn || fs2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(bm3d_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ms);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bm3d_filter_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs1);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bm3d_filter_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs2);
-    if (p.tensor) {
-        const size_t ts1 = filter_tc_smem(p, 1), ts2 = filter_tc_smem(p, 2);
-        if (ts2 > kSmemOptIn) return cudaErrorInvalidConfiguration;
-        const void* k1 = p.split ? (const void*)bm3d_filter_tc_kernel<1, true> : (const void*)bm3d_filter_tc_kernel<1, false>;
-        const void* k2 = p.split ? (const void*)bm3d_filter_tc_kernel<2, true> : (const void*)bm3d_filter_tc_kernel<2, false>;
-        const void* g1 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<1, true> : (const void*)bm3d_filter_tc_gated_kernel<1, false>;
-        const void* g2 = p.split ? (const void*)bm3d_filter_tc_gated_kernel<2, true> : (const void*)bm3d_filter_tc_gated_kernel<2, false>;
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts2);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts1);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts2);
-    }
-    return e;
+    constexpr size_t kSmemOptIn = 227 * 1024;
+    if (p.match_bytes > kSmemOptIn || filter_smem(p, 2) > kSmemOptIn) return cudaErrorInvalidConfiguration;
+    if (p.tensor && filter_tc_smem(p, 2) > kSmemOptIn) return cudaErrorInvalidConfiguration;
+    // The limit is a state of the kernel on the device, not of the plan: it is always
+    // the most that any plan may take, so that plans and threads agree on it.
+    static const void* const kernels[] = {
+        (const void*)bm3d_match_kernel, (const void*)bm3d_filter_kernel<1>, (const void*)bm3d_filter_kernel<2>,
+        (const void*)bm3d_filter_tc_kernel<1, true>, (const void*)bm3d_filter_tc_kernel<1, false>,
+        (const void*)bm3d_filter_tc_kernel<2, true>, (const void*)bm3d_filter_tc_kernel<2, false>,
+        (const void*)bm3d_filter_tc_gated_kernel<1, true>, (const void*)bm3d_filter_tc_gated_kernel<1, false>,
+        (const void*)bm3d_filter_tc_gated_kernel<2, true>, (const void*)bm3d_filter_tc_gated_kernel<2, false>};
+    for (const void* k : kernels)
+        if (const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
+            e != cudaSuccess)
+            return e;
+    return cudaSuccess;
 }
 
 cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16, void* scratch, cudaStream_t st,

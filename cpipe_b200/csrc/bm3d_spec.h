@@ -37,8 +37,9 @@ struct Bm3dPlan {
 // each image is denoised on its own (search windows stay inside it).
 int bm3d_plan(const cpipe_Bm3dSpecParams* p, int w, int h, Bm3dPlan* out, int batch = 1);
 
-// Sets the kernels' shared-memory limits for the plan (host-side; call
-// before capturing bm3d_run into a graph).
+// Raises the kernels' shared-memory limits on the current device to what any
+// plan may take, and refuses a plan that takes more (host-side; call before
+// capturing bm3d_run into a graph).
 cudaError_t bm3d_setup(const Bm3dPlan& plan);
 
 // RGBA in -> RGBA out (both binary16 when f16, else float32; alpha copied);

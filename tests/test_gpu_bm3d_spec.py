@@ -82,6 +82,25 @@ def test_bm3d_spec_windows_and_ties(cuda_device, h, w, kw, levels):
     compare(gpu_bm3d(x, blob).astype(np.float32), want, f"{w}x{h} {kw} levels {levels}")
 
 
+@pytest.mark.parametrize("graph", [True, False])
+def test_small_windows_leave_other_plans_their_shared_memory(cuda_device, graph):
+    """A kernel's shared-memory limit belongs to the device: a filter call and a chain of smaller windows, made between
+    a chain's creation and its runs, do not lower it."""
+    from cpipe_b200.chain import Chain, ChainConfig
+    cfg = ChainConfig.full_12mp(width=96, height=72, denoise="bm3d", stop_after=2, use_graph=graph)
+    raw = cfg.make_raw()
+    first = Chain(cfg)
+    x = noisy_rgba(clean_rgb(3, 40, 40), 0.03, 3)
+    for transform in ("tensor", "fp32", "tensor_fp16"):
+        gpu_bm3d(x, blobs.bm3d_spec(0.03, ns=3, nstep=1, transform=transform))
+    got = first.run_host(raw)
+    first.close()
+    alone = Chain(cfg)
+    want = alone.run_host(raw)
+    alone.close()
+    compare(got, want, "after smaller plans")
+
+
 def test_bm3d_spec_f32_buffers(cuda_device):
     clean = clean_rgb(5, 72, 88)
     x = noisy_rgba(clean, 0.03, 5, dtype=np.float32)
