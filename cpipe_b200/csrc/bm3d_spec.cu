@@ -25,7 +25,8 @@
 // multiply-adds, the library being built without contraction):
 //   bm3d_prep_kernel    RGBA -> Y,U,V planes + 8-bit matching luminance
 //   bm3d_match_kernel   block distances on the integer tensor cores, two passes
-//                       (a bound, then the candidates it lets through)
+//                       (a bound, then the candidates it lets through); small
+//                       windows: bm3d_match_each_kernel, a thread per reference
 //   bm3d_filter_kernel  one warp per group and channel: lane = (block, row
 //                       half); row DCT in registers, column DCT through a warp
 //                       shared buffer, Haar along the group with warp shuffles;
@@ -459,6 +460,122 @@ __global__ void __launch_bounds__(256, 2) bm3d_match_kernel(MatchArgs a) {
             const int widx = (int)(keys[m] & 2047U);
             const int dy = widx / a.ns - a.R, dx = widx % a.ns - a.R;
             out[1 + m] = ((uint32_t)(ry + dy) << 16) | (uint32_t)(rx + dx);
+            ++n;
+        }
+    }
+    a.cnt[ref] = (uint8_t)n;
+}
+
+// The same lists for small windows: a thread per reference visits its own
+// candidates only, where the warp's 8 x 4 references above share the union of
+// their windows (14 times a 5 x 5 window's pairs at step 3).  Distances with
+// byte-SIMD |a - b| and dp4a; a sorted register list keeps the 15 best keys.
+// The region of 16 x 16 references is staged as four byte-shifted word copies.
+constexpr int kMatchEachTile = 16;
+__global__ void __launch_bounds__(256) bm3d_match_each_kernel(MatchArgs a) {
+    extern __shared__ uint32_t s_w[];
+    const int wpr = a.wpr, plane = a.plane;  // words per staged row and per shifted copy
+    if (gated_off(a.gate)) return;
+    const int img = blockIdx.z, row0 = img * a.h;  // images are stacked in rows
+    const int i0 = blockIdx.x * kMatchEachTile, j0 = blockIdx.y * kMatchEachTile;
+    const int iL = min(i0 + kMatchEachTile - 1, a.nrx - 1), jL = min(j0 + kMatchEachTile - 1, a.nry - 1);
+    const int rx0 = max(0, refpos(i0, a.w, a.nstep) - a.R);
+    const int rx1 = min(a.w, refpos(iL, a.w, a.nstep) + a.R + 8);
+    const int ry0 = row0 + max(0, refpos(j0, a.h, a.nstep) - a.R);
+    const int ry1 = row0 + min(a.h, refpos(jL, a.h, a.nstep) + a.R + 8);
+    const int RW = rx1 - rx0, RH = ry1 - ry0;
+    // Copy s, row r, word k holds region bytes 4k+s .. 4k+s+3 (little endian).
+    for (int idx = threadIdx.x; idx < 4 * RH * wpr; idx += blockDim.x) {
+        const int s = idx / (RH * wpr), rem = idx - s * RH * wpr;
+        const int r = rem / wpr, k = rem - r * wpr;
+        const uint8_t* row = a.q + (size_t)(ry0 + r) * a.w + rx0;
+        const int c0 = 4 * k + s;
+        uint32_t word = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int cc = c0 + b;
+            word |= (cc < RW ? (uint32_t)row[cc] : 0U) << (8 * b);
+        }
+        s_w[s * plane + r * wpr + k] = word;
+    }
+    __syncthreads();
+    const int i = i0 + (int)(threadIdx.x % kMatchEachTile), j = j0 + (int)(threadIdx.x / kMatchEachTile);
+    if (i >= a.nrx || j >= a.nry) return;
+    const int x = refpos(i, a.w, a.nstep), y = row0 + refpos(j, a.h, a.nstep);
+    uint32_t rw[16];
+    {
+        const int c = x - rx0;
+        const uint32_t* p = s_w + (c & 3) * plane + (y - ry0) * wpr + (c >> 2);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            rw[2 * r] = p[r * wpr];
+            rw[2 * r + 1] = p[r * wpr + 1];
+        }
+    }
+    uint32_t keys[15];
+#pragma unroll
+    for (int m = 0; m < 15; ++m) keys[m] = 0xFFFFFFFFU;
+    const int ylo = max(row0, y - a.R), yhi = min(row0 + a.h - 8, y + a.R);
+    const int xlo = max(0, x - a.R), xhi = min(a.w - 8, x + a.R);
+    if (a.n2 > 1) {
+        // Columns of the search window outer, rows inner: the candidate's eight
+        // rows sit in a register ring (slot = row & 7, rows counted from ylo), so
+        // each candidate loads one new row.  Keys are unique (distance, window
+        // index), so the sorted list does not depend on the visiting order.
+        const int ny = yhi - ylo + 1;
+        for (int xx = xlo; xx <= xhi; ++xx) {
+            const int c = xx - rx0;
+            const uint32_t* colp = s_w + (c & 3) * plane + (ylo - ry0) * wpr + (c >> 2);
+            const uint32_t wcol = (uint32_t)((ylo - y + a.R) * a.ns + a.R - x + xx);
+            uint32_t cw[8][2];
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {
+                cw[r][0] = colp[r * wpr];
+                cw[r][1] = colp[r * wpr + 1];
+            }
+            cw[7][0] = cw[7][1] = 0U;
+            for (int y0 = 0; y0 < ny; y0 += 8) {
+                const uint32_t* rp = colp + (y0 + 7) * wpr;
+#pragma unroll
+                for (int st = 0; st < 8; ++st) {
+                    if (y0 + st < ny) {
+                        cw[(st + 7) & 7][0] = rp[st * wpr];
+                        cw[(st + 7) & 7][1] = rp[st * wpr + 1];
+                        uint32_t d = 0;
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) {
+                            const uint32_t a0 = __vabsdiffu4(rw[2 * r], cw[(st + r) & 7][0]);
+                            d = __dp4a(a0, a0, d);
+                            const uint32_t a1 = __vabsdiffu4(rw[2 * r + 1], cw[(st + r) & 7][1]);
+                            d = __dp4a(a1, a1, d);
+                        }
+                        const int yy = ylo + y0 + st;
+                        if (d <= a.dthr && (xx != x || yy != y)) {
+                            uint32_t key = (d << 11) | (wcol + (uint32_t)((y0 + st) * a.ns));
+                            if (key < keys[14]) {
+#pragma unroll
+                                for (int m = 0; m < 15; ++m) {
+                                    const uint32_t lo = min(keys[m], key);
+                                    key = max(keys[m], key);
+                                    keys[m] = lo;
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    const long long ref = ((long long)img * a.nry + j) * a.nrx + i;
+    uint32_t* out = a.list + ref * 16;
+    out[0] = ((uint32_t)y << 16) | (uint32_t)x;
+    int n = 1;
+#pragma unroll
+    for (int m = 0; m < 15; ++m) {
+        if (m < a.n2 - 1 && keys[m] != 0xFFFFFFFFU) {
+            const int widx = (int)(keys[m] & 2047U);
+            const int dy = widx / a.ns - a.R, dx = widx % a.ns - a.R;
+            out[1 + m] = ((uint32_t)(y + dy) << 16) | (uint32_t)(x + dx);
             ++n;
         }
     }
@@ -1201,6 +1318,31 @@ size_t match_layout(Bm3dPlan& p, int tile) {
     return sizeof(uint32_t) *
            (4 * (size_t)p.mplane + (size_t)p.mepitch * (p.mwin - 7) + (size_t)(tile * tile) * kMatchStride);
 }
+// The same of the form with a thread per reference.
+size_t match_each_layout(Bm3dPlan& p) {
+    p.mtile = kMatchEachTile;
+    p.mwin = (kMatchEachTile - 1) * p.nstep + 2 * p.R + 8;
+    p.mwpr = (p.mwin + 3) / 4 + 1;
+    p.mplane = p.mwin * p.mwpr;
+    p.mepitch = 0;
+    return sizeof(uint32_t) * 4 * (size_t)p.mplane;
+}
+// The smallest window that the matching on the tensor cores takes.  Its warps
+// share the union of 8 x 4 references' windows, so small windows and large steps
+// waste its products, and a thread per reference is faster; with CTAs for less
+// than a quarter of the SMs that thread's serial walk counts instead.  Stage 1
+// with either form (us; 320 x 240 has few, 2016 x 1512 many):
+//   window, step           9, 3   21, 3  27, 3  33, 4  39, 4  39, 6  45, 6  39, 8
+//   few:  tensor cores     162    207    223    257    281    314    330    338
+//         thread           112    180    233    286    350    347    422    351
+//   many: tensor cores     2542   2840   2930   2292   2557   1500   1682   1417
+//         thread           2282   2688   2942   2029   2372   1301   1648   1023
+// (Where the two are close on large frames the line keeps to the tensor cores.)
+int match_from(const Bm3dPlan& p) {
+    constexpr int few[8] = {21, 27, 27, 33, 33, 33, 39, 39}, many[8] = {21, 27, 27, 39, 39, 39, 47, 47};
+    const int ctas = ((p.nrx + kMatchEachTile - 1) / kMatchEachTile) * ((p.nry + kMatchEachTile - 1) / kMatchEachTile);
+    return (ctas * p.batch < kSmCount / 4 ? few : many)[p.nstep - 1];
+}
 // Row pitch of the tensor-core form's footprint planes: at least fw and 4 mod
 // 32 (column loads of eight columns x two rows, and atomics of eight rows x
 // four columns, fall in 32 different banks).
@@ -1261,8 +1403,10 @@ int bm3d_plan(const cpipe_Bm3dSpecParams* p, int w, int h, Bm3dPlan* out, int ba
     q.ntx = (q.nrx + kRefTile - 1) / kRefTile;
     q.nty = (q.nry + kRefTile - 1) / kRefTile;
     // 16 x 16 references a CTA share a region best; the largest windows and steps need 8 x 8
-    q.match_bytes = match_layout(q, 16);
-    if (q.match_bytes > 227 * 1024) q.match_bytes = match_layout(q, 8);
+    q.match_each = n2 == 1 || q.ns < match_from(q);  // (n2 = 1: nothing to search)
+    if (q.match_each) q.match_bytes = match_each_layout(q);
+    else q.match_bytes = match_layout(q, 16);
+    if (!q.match_each && q.match_bytes > 227 * 1024) q.match_bytes = match_layout(q, 8);
     const size_t npx = (size_t)w * h * batch, nref = (size_t)q.nrx * q.nry * batch;
     size_t o = 0;
     q.off_yuv = o;
@@ -1289,7 +1433,7 @@ cudaError_t bm3d_setup(const Bm3dPlan& p) {
     // The limit is a state of the kernel on the device, not of the plan: it is always
     // the most that any plan may take, so that plans and threads agree on it.
     static const void* const kernels[] = {
-        (const void*)bm3d_match_kernel, (const void*)bm3d_filter_kernel<1>, (const void*)bm3d_filter_kernel<2>,
+        (const void*)bm3d_match_kernel, (const void*)bm3d_match_each_kernel, (const void*)bm3d_filter_kernel<1>, (const void*)bm3d_filter_kernel<2>,
         (const void*)bm3d_filter_tc_kernel<1, true>, (const void*)bm3d_filter_tc_kernel<1, false>,
         (const void*)bm3d_filter_tc_kernel<2, true>, (const void*)bm3d_filter_tc_kernel<2, false>,
         (const void*)bm3d_filter_tc_gated_kernel<1, true>, (const void*)bm3d_filter_tc_gated_kernel<1, false>,
@@ -1364,7 +1508,8 @@ cudaError_t bm3d_run(const Bm3dPlan& p, const Img& in, const Img& out, bool f16,
     for (int stage = 1; stage <= p.stages; ++stage) {
         bm3d_zero_kernel<<<kSmCount * 8, 256, 0, st>>>(acc, 6 * npx, gate);
         ma.dthr = p.dthr[stage - 1];
-        bm3d_match_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
+        if (p.match_each) bm3d_match_each_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
+        else bm3d_match_kernel<<<mgrid, p.mtile * p.mtile, p.match_bytes, st>>>(ma);
         if (p.tensor && gate) {
             const int tiles = p.ntx * p.nty * 3 * p.batch, g = std::min(tiles, kSmCount * (stage == 1 ? 4 : 3));
             if (p.split) {

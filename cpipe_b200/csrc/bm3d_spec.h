@@ -26,6 +26,7 @@ struct Bm3dPlan {
     // match kernel: references per CTA edge, region edge bound, pitches in words, shared memory
     int mtile = 0, mwin = 0, mwpr = 0, mplane = 0, mepitch = 0;
     size_t match_bytes = 0;
+    bool match_each = false;  // small windows: matching with a thread per reference
     bool copy = false;       // image below 8x8 or sigma <= 0: output = input
     bool tensor = true;      // transforms on the tensor cores or FP32 CUDA cores
     bool split = true;       // tensor cores: FP16 hi/lo split products (else single FP16 products)
