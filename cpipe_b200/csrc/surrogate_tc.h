@@ -9,6 +9,7 @@ namespace cpb {
 struct TcNetArgs {
     int n, h, w;               // frames and their size
     int strips;                // columns are walked in this many strips (set by tc_net)
+    int bands, band_rows;      // narrow frames: bands of rows side by side, and a band's rows (set by tc_net)
     const void* rgba;          // dense RGBA frames [n][h][w][4]: the network's input and the residual's base
     void* out;                 // back half: the denoised frames (may be rgba)
     const float* ab;           // front half: n (a, b) noise-model pairs

@@ -72,6 +72,42 @@ def test_tcgen05_strips_match_mma(cuda_device, n, h, w):
     sg.close()
 
 
+# frames of at most 63 columns and more than 1184 rows in all go by bands of rows side by side: just below and above that
+# line, two bands to 64 of them (63, 62, 42 .. 1 columns), the widest that fits (63) and the first that does not (64),
+# bands that end inside a frame and on the zeros after it, many frames, of one row too
+@pytest.mark.parametrize("n,h,w", [(1, 1184, 2), (1, 1185, 2), (600, 1, 20), (3, 431, 62), (1, 2500, 63), (1, 3000, 64),
+                                   (2, 1700, 42), (1, 5000, 31), (100, 16, 16), (7, 1300, 16), (1, 9001, 9),
+                                   (2, 19000, 2), (1, 76000, 1), (25, 59, 5)])
+@pytest.mark.parametrize("f16", [True, False])
+def test_tcgen05_bands_match_mma(cuda_device, n, h, w, f16):
+    rng = np.random.default_rng(h * 1000 + w)
+    x = rng.uniform(0.02, 0.95, (n, h, w, 4)).astype(np.float16 if f16 else np.float32)
+    ab = np.tile(np.array([(4e-3, 4e-5), (1e-3, 1e-5), (8e-3, 9e-5)], np.float32), (n // 3 + 1, 1))[:n]
+    params = [(W, (b + rng.normal(0, 0.02, b.shape)).astype(np.float32)) for W, b in S.init_params(n + h)]
+    params[-1] = (params[-1][0] * 10.0, params[-1][1])
+    sg = S.Surrogate(S.to_blob(params))
+    tc, mma = run(sg, "tcgen05", x, ab, f16), run(sg, "mma", x, ab, f16)
+    np.testing.assert_array_equal(tc[..., 3], x[..., 3].astype(np.float32))
+    close(tc[..., :3], mma[..., :3], f"tcgen05 vs mma {n}x{h}x{w}")
+    sg.close()
+
+
+def test_narrow_frames_fill_the_products(cuda_device):
+    """A pixel of a 16-column frame costs at most 2.5 times one of a wide frame (a strip of 16 columns in products of
+    128 pixels cost six times as much)."""
+    sg = S.Surrogate(S.to_blob(S.init_params(1)))
+    d = [S.DeviceArray(1200000 * 8), S.DeviceArray(1200000 * 8)]
+
+    def ms(w, h):
+        return min(sum(sg.profile(d[0].ptr, d[1].ptr, 1, w, h, [(1e-3, 1e-5)])) for _ in range(5))
+
+    d[0].upload(np.zeros((1200000, 4), np.float16))
+    wide, narrow = ms(1200, 1000), ms(16, 75000)
+    print(f"1.2 MP: 1200 columns {wide:.3f} ms, 16 columns {narrow:.3f} ms")
+    assert narrow <= 2.5 * wide
+    sg.close()
+
+
 def test_tcgen05_float32_frames(cuda_device):
     rng = np.random.default_rng(7)
     x = rng.uniform(0.02, 0.95, (1, 24, 40, 4)).astype(np.float32)
