@@ -1565,9 +1565,10 @@ __device__ __forceinline__ int next_item(const Frame* __restrict__ frames, const
 // -> 2225 us a batch against tiles; two CTAs an SM at 128 registers, with a few spilled, as the frame's
 // parameters come from shared memory.)
 constexpr int kItemRows = 24;
-template <int ALGO>
-__global__ void __launch_bounds__(256, 2) batch_raw_kernel(const Frame* __restrict__ frames,
-                                                        const int* __restrict__ prefix, int n) {
+// STRIPS: some frame of the batch goes by strips.  A batch without has a kernel of its own: in the
+// strips' registers its tiles ran at two CTAs an SM (eight frames of 0.35 MP: 316 us a batch, 285 apart).
+template <int ALGO, bool STRIPS>
+__device__ __forceinline__ void batch_raw_items(const Frame* __restrict__ frames, const int* __restrict__ prefix, int n) {
     __shared__ int s_prefix[kMaxFrames + 1];
     __shared__ Frame s_f;
     for (int i = threadIdx.x; i <= n; i += blockDim.x) s_prefix[i] = prefix[i];
@@ -1576,7 +1577,7 @@ __global__ void __launch_bounds__(256, 2) batch_raw_kernel(const Frame* __restri
     for (int t = blockIdx.x; t < s_prefix[n]; t += gridDim.x) {
         const int local = next_item(frames, s_prefix, n, t, &s_f, &cur);
         const int tx = local % s_f.t1x, ty = local / s_f.t1x;
-        if constexpr (ALGO != 0) {
+        if constexpr (STRIPS) {
             if (s_f.strip >= 0) {
                 const int ys = (8 * ty + (int)(threadIdx.x >> 5)) * kItemRows;
                 if (ys < s_f.bayer.h) {
@@ -1591,6 +1592,15 @@ __global__ void __launch_bounds__(256, 2) batch_raw_kernel(const Frame* __restri
                                        tx * kDmTW, ty * kDmTH);
         __syncthreads();
     }
+}
+template <int ALGO>
+__global__ void __launch_bounds__(256) batch_raw_kernel(const Frame* __restrict__ frames, const int* __restrict__ prefix, int n) {
+    batch_raw_items<ALGO, false>(frames, prefix, n);
+}
+template <int ALGO>
+__global__ void __launch_bounds__(256, 2)
+    batch_raw_strip_kernel(const Frame* __restrict__ frames, const int* __restrict__ prefix, int n) {
+    batch_raw_items<ALGO, true>(frames, prefix, n);
 }
 
 template <bool WARP>
@@ -1651,6 +1661,7 @@ struct cpipe_cuda_batch {
     int* d_prefix = nullptr;  // three arrays of n + 1
     int n = 0, algo = 1, radius = 2;
     bool warp = false;
+    bool strips = false;  // some frame's stage 1 goes by strips
     int per_sm[3] = {2, 8, 3};  // persistent CTAs per SM for the three stages (autotuned)
     int rows2 = cpb::batch::kK2Rows;  // rows per stage-2 work item (autotuned)
     int denoise_mode = 0;             // 0: the reference's 2x2 blend in K3; 1 / 2: BM3D / the network between K2 and K3
@@ -1676,7 +1687,9 @@ int batch_launch_stage(cpipe_cuda_batch* b, int stage, cudaStream_t st, bool tim
     const int* pf = b->d_prefix + stage * (b->n + 1);
     if (stage == 0) {
         if (b->algo == 0) cpb::batch::batch_raw_kernel<0><<<grid, 256, 0, st>>>(b->d_frames, pf, b->n);
+        else if (b->algo == 1 && b->strips) cpb::batch::batch_raw_strip_kernel<1><<<grid, 256, 0, st>>>(b->d_frames, pf, b->n);
         else if (b->algo == 1) cpb::batch::batch_raw_kernel<1><<<grid, 256, 0, st>>>(b->d_frames, pf, b->n);
+        else if (b->strips) cpb::batch::batch_raw_strip_kernel<2><<<grid, 256, 0, st>>>(b->d_frames, pf, b->n);
         else cpb::batch::batch_raw_kernel<2><<<grid, 256, 0, st>>>(b->d_frames, pf, b->n);
     } else if (stage == 1) {
         if (b->warp) cpb::batch::batch_color_kernel<true><<<grid, 128, 0, st>>>(b->d_frames, pf, b->n);
@@ -1846,11 +1859,13 @@ cpipe_cuda_batch* cpipe_cuda_batch_create(const cpipe_cuda_chain_config* cfgs, s
         f.t3x = (w + kCTW - 1) / kCTW;
         b->frames.push_back(f);
     }
-    // Bayer frames by strips where the batch makes some items for every SM (two from 3.6 MP on)
+    // Bayer frames by strips where the batch makes some items for every SM (two from 3.6 MP on):
+    // one frame of 1 MP 104 us by strips, 98 by tiles; of 2 MP 174 and 175; 8 of 0.35 MP 294 and 285;
+    // 4 of 1.1 MP 367 and 371; 8 of 1 to 6 MP 1560 and 1620
     if (b->algo != 0 && tiles >= 24LL * kSmCount)
         for (Frame& f : b->frames) {
             f.strip = cpb::strip_phase(f.raw.cfa);
-            if (f.strip >= 0) f.t1x = (f.mid0.w + kStrip - 1) / kStrip;
+            if (f.strip >= 0) f.t1x = (f.mid0.w + kStrip - 1) / kStrip, b->strips = true;
         }
     if (cudaMalloc(&b->d_frames, sizeof(Frame) * n) != cudaSuccess ||
         cudaMalloc(&b->d_prefix, sizeof(int) * 3 * (n + 1)) != cudaSuccess ||
