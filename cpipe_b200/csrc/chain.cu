@@ -263,6 +263,9 @@ bool launch_raw_strips(const Img& raw, const Img& out, const RawParams& p, cudaS
     // rows a warp: the six rows walked twice cost less the more there are, while there are warps
     // enough for the chip (50 MP, AMaZE: 36 rows 280 us, 24 rows 299, 12 rows 359; 12 MP, RCD: 84, 84, 95)
     const unsigned cols = (unsigned)((raw.w + kStrip - 1) / kStrip);
+    // two strips where one tile is wide enough (57 to 64 columns) cost more than it: 57 x 40000 57 us
+    // against 51 (56 x 40000, 113 x 10000 and all wider frames are level or faster by strips)
+    if (cols >= 2U * ((raw.w + kDmTW - 1) / kDmTW)) return false;
     auto warps = [&](int R) { return (long long)cols * ((raw.h + R - 1) / R); };
     const int R = warps(36) >= kSmCount * 64 ? 36 : warps(24) >= kSmCount * 12 ? 24 : 12;
     const dim3 g(cols, (unsigned)((raw.h + R * kStripWarps - 1) / (R * kStripWarps)));
