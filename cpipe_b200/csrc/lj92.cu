@@ -344,7 +344,7 @@ struct LjRun {
         const uint32_t f = runs[ph * kLut + (w >> (32 - kLutBits))];
         uint32_t total = whole ? f & 31u : f >> 11, count = whole ? (f >> 5) & 15u : 1u;
         uint32_t after = whole ? (f >> 9) & 3u : x.step(ph);
-        if (f == 0) {
+        if (f == 0 && on) {
             bool ok = true;
             total = lj_total(x, w, 0, ph, ok);
             count = ok;
@@ -612,12 +612,16 @@ __global__ void __launch_bounds__(kChunksPerCta) lj_cand_kernel(const SegDev* __
         // Where the tables give the codes in play the same lengths (a flat
         // stretch, a padded tile edge) a path can sit on the true boundaries one
         // component off for any length.
-        const bool two = c > 0 && !x.shared;
-        LjRun b = {two ? a.pos : ce, x.step(a.ph), 0};
-        const LjRun a0 = a, b0 = b;
-        lj_run_pair(x, runs, br, ce, a, b);
+        const LjRun a0 = a;
+        if (x.shared) {
+            a.to(x, runs, br, ce);
+        } else {
+            LjRun b = {c > 0 ? a.pos : ce, x.step(a.ph), 0};
+            const LjRun b0 = b;
+            lj_run_pair(x, runs, br, ce, a, b);
+            if (c > 0) p1 = lj_cand(b0, b);
+        }
         p0 = lj_cand(a0, a);
-        if (two) p1 = lj_cand(b0, b);
     }
     first[2 * threadIdx.x] = p0;
     first[2 * threadIdx.x + 1] = p1;
