@@ -789,7 +789,7 @@ def b200_arm(args):
         "reference_computation_chain": {"ms_per_frame": round(ref_value, 4),
                                         "note": "denoise.bm3d as the reference computes it (2x2 box blend)",
                                         "per_stage_ms": {k: round(v, 4) for k, v in ref_stages.items()}},
-        "surrogate_layer_ms": [round(v, 4) for v in layer_ms],
+        "surrogate_kernel_ms": {"layers 0-3": round(layer_ms[1], 4), "layers 4-7": round(layer_ms[5], 4)},
         "roofline": {"bound": "tensor", "kernel": "sg_tc_net_kernel (tcgen05, two launches of four 3x3 conv layers)",
                      "achieved": round(achieved_tf, 1), "peak": peak_tf, "peak_kind": peak_kind,
                      "unit": "TFLOP/s", "frac": round(achieved_tf / peak_tf, 4),

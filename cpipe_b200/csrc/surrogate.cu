@@ -690,7 +690,7 @@ static cudaError_t infer(SurrogateNet* s, const void* in, void* out, int n, int 
     cudaError_t e = ensure_acts(s, px, false);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[0], st);
-    if (s->use_tc) {  // two kernels of four layers; the events between layers mark the kernel's end
+    if (s->use_tc) {  // two kernels of four layers, each timed at its first layer
         TcNetArgs t{};
         t.n = n;
         t.h = h;
@@ -865,15 +865,11 @@ int cpipe_surrogate_profile(cpipe_surrogate* s, const void* d_in, void* d_out, i
     if (status == CPIPE_OK && e == cudaSuccess) e = cudaEventSynchronize(ev[kLayers + 1]);
     if (status == CPIPE_OK && e == cudaSuccess) {
         for (int k = 0; k <= kLayers; ++k) cudaEventElapsedTime(&ms[k], ev[k], ev[k + 1]);
-        if (s->net->use_tc)  // a kernel's four layers share its time by their multiply-adds
-            for (int half = 0; half < 2; ++half) {
-                float* t = ms + 1 + 4 * half;
-                const float sum = t[0] + t[1] + t[2] + t[3];
-                float macs = 0.0F;
-                for (int p = 0; p < 4; ++p) macs += (float)(cin_real(4 * half + p) * cout_real(4 * half + p));
-                for (int p = 0; p < 4; ++p)
-                    t[p] = sum * (float)(cin_real(4 * half + p) * cout_real(4 * half + p)) / macs;
-            }
+        if (s->net->use_tc) {  // (the events behind a kernel are microseconds apart)
+            ms[0] = 0.0F;
+            for (int k = 2; k <= kLayers; ++k)
+                if (k != 5) ms[k] = 0.0F;
+        }
     }
     for (auto& x : ev)
         if (x) cudaEventDestroy(x);

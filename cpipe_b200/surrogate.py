@@ -180,7 +180,8 @@ class Surrogate:
             raise CpipeError(st, "surrogate_check " + A.lib().cpipe_cuda_last_error().decode())
 
     def profile(self, d_in, d_out, n, width, height, noise_ab, f16=True, stream=None):
-        """Per-kernel times (ms) of one denoise: [input map, layer 0, ..., layer 7]."""
+        """Times (ms) of one denoise: [input map, layer 0, ..., layer 7].  The tcgen05 engine's two kernels (input map
+        and layers 0-3; layers 4-7) stand at layers 0 and 4, the other places are 0."""
         keep, p = _ab(noise_ab)
         ms = (C.c_float * 9)()
         st = A.lib().cpipe_surrogate_profile(self._h, d_in, d_out, n, width, height, int(f16), p, ms, stream)

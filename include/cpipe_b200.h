@@ -415,9 +415,9 @@ int cpipe_surrogate_set_engine(cpipe_surrogate* s, int engine);
  * wait inside a tcgen05 kernel ran out since creation. */
 int cpipe_surrogate_check(cpipe_surrogate* s);
 /* One denoise with CUDA events between its kernels: ms[0] the input map,
- * ms[1 + l] layer l (l = 0..7).  The tcgen05 engine runs layers 0-3 (with the
- * input map, so ms[0] is 0) and 4-7 in one kernel each: the layers of a kernel
- * share its time by their multiply-adds.  Waits for the stream. */
+ * ms[1 + l] layer l (l = 0..7).  The tcgen05 engine runs the input map and
+ * layers 0-3, and layers 4-7, in one kernel each: ms[1] and ms[5] are their
+ * times, the other places 0.  Waits for the stream. */
 int cpipe_surrogate_profile(cpipe_surrogate* s, const void* d_in, void* d_out, int n, int width, int height, int f16,
                             const float* noise_ab, float ms[9], void* stream);
 /* One step on a batch: forward, mean-squared-error loss against the target,

@@ -108,6 +108,18 @@ def test_narrow_frames_fill_the_products(cuda_device):
     sg.close()
 
 
+def test_profile_reports_what_was_timed(cuda_device):
+    """The tcgen05 engine has two kernels: two times.  The mma.sync engine has nine."""
+    sg = S.Surrogate(S.to_blob(S.init_params(1)))
+    x = np.full((2, 60, 150, 4), 0.5, np.float16)
+    d = [S.DeviceArray(x.nbytes).upload(x), S.DeviceArray(x.nbytes)]
+    for engine, places in (("tcgen05", [1, 5]), ("mma", list(range(9)))):
+        sg.set_engine(engine)
+        ms = sg.profile(d[0].ptr, d[1].ptr, 2, 150, 60, [(1e-3, 1e-5)] * 2)
+        assert [k for k, v in enumerate(ms) if v != 0.0] == places, (engine, ms)
+    sg.close()
+
+
 def test_tcgen05_float32_frames(cuda_device):
     rng = np.random.default_rng(7)
     x = rng.uniform(0.02, 0.95, (1, 24, 40, 4)).astype(np.float32)
