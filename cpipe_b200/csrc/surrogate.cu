@@ -554,8 +554,9 @@ struct SurrogateNet {
     bool use_tc = true;          // inference on tcgen05 (else the mma.sync kernels)
     int step = 0;
     // activations for a batch of n x h x w
-    long long act_px = 0;
-    bf16* d_act = nullptr;       // a0 (8 ch) then a1..a7 (32 ch)
+    size_t act_elems = 0;        // of d_act
+    long long train_px = 0;      // pixels that the buffers are laid out for a training step of (0: inference)
+    bf16* d_act = nullptr;       // training: a0 (8 ch) then a1..a7 (32 ch); inference: ensure_acts
     bf16* d_g[2] = {nullptr, nullptr};  // gradient ping-pong (32 ch)
     bf16* d_gout = nullptr;             // dLoss/dOut (8 ch)
 };
@@ -598,18 +599,19 @@ static void free_acts(SurrogateNet* s) {
     cudaFree(s->d_g[1]);
     cudaFree(s->d_gout);
     s->d_act = s->d_g[0] = s->d_g[1] = s->d_gout = nullptr;
-    s->act_px = 0;
+    s->act_elems = 0;
+    s->train_px = 0;
 }
 
+// Activations for a training step (every layer's, and the gradients), or for
+// inference: the tcgen05 engine keeps one hidden activation, the mma.sync engine
+// the input map and two.  Inference keeps a larger allocation: the buffers are
+// laid out by the call's pixel count inside it (frames of a batch share one network).
 static cudaError_t ensure_acts(SurrogateNet* s, long long px, bool training) {
-    const long long need = training ? px : -px;  // training needs every activation and the gradients
-    if (s->act_px == need) return cudaSuccess;
-    // inference keeps a larger allocation: the layer buffers are laid out by
-    // the call's pixel count inside it (frames of a batch share one network)
-    if (!training && s->act_px < 0 && -s->act_px >= px) return cudaSuccess;
-    free_acts(s);
     const size_t a0 = (size_t)px * 8, hid = (size_t)px * kCh;
-    const size_t acts = training ? a0 + 7 * hid : a0 + 2 * hid;
+    const size_t acts = training ? a0 + 7 * hid : s->use_tc ? hid : a0 + 2 * hid;
+    if (training ? s->train_px == px : s->train_px == 0 && s->act_elems >= acts) return cudaSuccess;
+    free_acts(s);
     cudaError_t e = cudaMalloc(&s->d_act, acts * sizeof(bf16));
     if (e == cudaSuccess && training) e = cudaMalloc(&s->d_g[0], hid * sizeof(bf16));
     if (e == cudaSuccess && training) e = cudaMalloc(&s->d_g[1], hid * sizeof(bf16));
@@ -618,7 +620,8 @@ static cudaError_t ensure_acts(SurrogateNet* s, long long px, bool training) {
         free_acts(s);
         return e;
     }
-    s->act_px = need;
+    s->act_elems = acts;
+    s->train_px = training ? px : 0;
     return cudaSuccess;
 }
 

@@ -120,6 +120,34 @@ def test_profile_reports_what_was_timed(cuda_device):
     sg.close()
 
 
+def test_workspace_follows_the_engine(cuda_device):
+    """Inference on tcgen05 keeps one hidden activation, 64 bytes a pixel; the mma.sync engine's 144 are allocated when
+    it is asked for, a training step's too, and each engine's output stays its own."""
+    import torch
+    w, h = 2048, 2048
+    rng = np.random.default_rng(9)
+    x = np.tile(rng.uniform(0.02, 0.95, (1, 64, w, 4)), (1, h // 64, 1, 1)).astype(np.float16)
+    ab = np.array([(4e-3, 4e-5)], np.float32)
+    params = S.init_params(4)
+    params[-1] = (params[-1][0] * 10.0, params[-1][1])
+    sg = S.Surrogate(S.to_blob(params))
+    small = x[:, :16, :16].copy()
+    run(sg, "tcgen05", small, ab)  # (the kernels' own setup)
+    dev = [S.DeviceArray(x.nbytes).upload(x), S.DeviceArray(x.nbytes)]
+    before = torch.cuda.mem_get_info()[0]
+    sg.denoise(dev[0].ptr, dev[1].ptr, 1, w, h, ab)
+    sg.check()
+    used = before - torch.cuda.mem_get_info()[0]
+    assert 60 * w * h <= used <= 72 * w * h, used / (w * h)
+    tc = dev[1].download(x.shape, x.dtype).astype(np.float32)
+    mma = run(sg, "mma", x, ab)
+    close(tc[..., :3], mma[..., :3], "after regrowing")
+    d16 = S.DeviceArray(small.nbytes).upload(small)
+    sg.train_step(d16.ptr, d16.ptr, ab, 1, 16, 16, 0.0, update=False)
+    np.testing.assert_array_equal(run(sg, "tcgen05", x, ab), tc)
+    sg.close()
+
+
 def test_tcgen05_float32_frames(cuda_device):
     rng = np.random.default_rng(7)
     x = rng.uniform(0.02, 0.95, (1, 24, 40, 4)).astype(np.float32)
