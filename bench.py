@@ -611,7 +611,7 @@ def qbc_50mp(weights):
         out[key] = round(ms.value / 3, 3)
         if mode == "surrogate":
             f, fb, worst = ch.denoise_stats()
-            out["spot_check"] = {"frames": f, "fallbacks_to_bm3d": fb, "worst_tile_psnr_db": round(worst, 2)}
+            out["spot_check"] = {"frames": f, "fallbacks_to_bm3d": fb, "worst_tile_psnr_db": B.db(worst)}
         ch.close()
     L.cpipe_cuda_device_free(d_raw)
     L.cpipe_cuda_device_free(d_out)
@@ -629,6 +629,7 @@ def b200_arm(args):
         dist.init_process_group("nccl", timeout=__import__("datetime").timedelta(seconds=120))
     from cpipe_b200 import _abi as A
     from cpipe_b200 import surrogate as S
+    from cpipe_b200.batch import db
     from cpipe_b200.chain import Chain, ChainConfig
     from cpipe_b200.roofline import node_roofline
     L = A.lib()
@@ -785,7 +786,7 @@ def b200_arm(args):
         "psnr_denoiser_vs_bm3d_db": round(den_psnr, 2),
         "spot_check": {"tiles_per_frame": cfg.spot_tiles, "tile": "256x256", "min_psnr_db": cfg.spot_min_psnr_db,
                        "frames": spot_frames, "fallbacks_to_bm3d": spot_fallbacks,
-                       "worst_tile_psnr_db": round(spot_worst, 2)},
+                       "worst_tile_psnr_db": db(spot_worst)},
         "reference_computation_chain": {"ms_per_frame": round(ref_value, 4),
                                         "note": "denoise.bm3d as the reference computes it (2x2 box blend)",
                                         "per_stage_ms": {k: round(v, 4) for k, v in ref_stages.items()}},

@@ -123,6 +123,11 @@ class Batch:
         return list(ms)
 
 
+def db(v):
+    """A PSNR for a JSON line, which has no infinities."""
+    return round(v, 2) if math.isfinite(v) else None
+
+
 def measure(n=64, reps=5, seed=0x5EED0004, **chain_kw):
     """Aggregate MP/s of the batched form; per-frame latency (p50 / p99) both
     inside the batched launch (completion times on the device clock) and for
@@ -158,12 +163,17 @@ def measure(n=64, reps=5, seed=0x5EED0004, **chain_kw):
     per_sm, rows2 = batch.schedule()
     stats = None
     if chain_kw.get("denoise") == "surrogate":
-        fr, fb, worst = 0, 0, float("inf")
+        fr, fb, worst, broken = 0, 0, float("inf"), 0
         for i in range(n):
             f_, fb_, w_ = C.c_uint32(), C.c_uint32(), C.c_float()
             L.cpipe_cuda_chain_denoise_stats(batch.frame_chain(i), C.byref(f_), C.byref(fb_), C.byref(w_))
-            fr, fb, worst = fr + f_.value, fb + fb_.value, min(worst, w_.value)
-        stats = {"frames": fr, "fallbacks_to_bm3d": fb, "worst_tile_psnr_db": round(worst, 2)}
+            fr, fb = fr + f_.value, fb + fb_.value
+            if w_.value == float("-inf"):  # a tile's error was not finite
+                broken += 1
+            else:
+                worst = min(worst, w_.value)
+        stats = {"frames": fr, "fallbacks_to_bm3d": fb, "worst_tile_psnr_db": db(worst),
+                 "frames_of_the_mix_with_a_non_finite_tile": broken}
     total_mp = sum(cfg.width * cfg.height for cfg, _ in frames) / 1e6
     lat = []
     for i, (cfg, _) in enumerate(frames):

@@ -377,8 +377,8 @@ int cpipe_cuda_chain_run_host_frames(cpipe_cuda_chain* chain, const uint16_t* co
 int cpipe_cuda_chain_set_profiling(cpipe_cuda_chain* chain, int enable);
 int cpipe_cuda_chain_profile(cpipe_cuda_chain* chain, double ms_per_stage[4], int* frames);
 /* Spot-check counters since creation (denoise_mode 2): frames checked, frames
- * that fell back to BM3D, and the lowest tile PSNR seen (dB).  Waits for the
- * device. */
+ * that fell back to BM3D, and the lowest tile PSNR seen (dB; -infinity when a
+ * tile's error was not finite, which also falls back).  Waits for the device. */
 int cpipe_cuda_chain_denoise_stats(cpipe_cuda_chain* chain, uint32_t* frames, uint32_t* fallbacks,
                                    float* worst_tile_psnr_db);
 /* Seeded synthetic raw frame on the device (uint16, width x height): linear

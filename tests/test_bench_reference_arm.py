@@ -44,3 +44,10 @@ def test_reference_arm_other_ranks_do_no_work(monkeypatch):
     with contextlib.redirect_stdout(out):
         assert bench.reference_arm(argparse.Namespace(gpus=2, steps=2, warmup=1)) == 0
     assert out.getvalue() == ""
+
+
+def test_psnr_of_a_json_line():
+    """A frame with a non-finite tile reports -infinity, a perfect one +infinity; JSON has neither."""
+    from cpipe_b200.batch import db
+    assert db(42.534) == 42.53
+    assert json.loads(json.dumps([db(float("-inf")), db(float("inf"))], allow_nan=False)) == [None, None]
