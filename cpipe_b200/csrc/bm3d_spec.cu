@@ -21,20 +21,26 @@
 //             num / den and keeps FP32 from overflowing
 //   aggregate weight x Kaiser(beta) 8x8 window; estimate = num / den
 //
-// Kernels (all FP32 on the CUDA cores; the transforms use explicit fused
-// multiply-adds, the library being built without contraction):
+// Kernels:
 //   bm3d_prep_kernel    RGBA -> Y,U,V planes + 8-bit matching luminance
 //   bm3d_match_kernel   block distances on the integer tensor cores, two passes
 //                       (a bound, then the candidates it lets through); small
 //                       windows: bm3d_match_each_kernel, a thread per reference
-//   bm3d_filter_kernel  one warp per group and channel: lane = (block, row
-//                       half); row DCT in registers, column DCT through a warp
-//                       shared buffer, Haar along the group with warp shuffles;
-//                       aggregation into a shared-memory footprint of the 8x8
-//                       reference tile, then added to the frame accumulators.
-//                       Tiles are launched in P x P phases so that tiles of one
-//                       launch have disjoint footprints: the flush is a plain
-//                       read-modify-write, no global atomics.
+//   bm3d_filter_tc_kernel
+//                       the default filter: one warp per group and channel, the
+//                       separable DCTs on the FP16 tensor cores (hi/lo split, or
+//                       single products for the spot check), the Haar in
+//                       registers; one launch over all tiles, whose footprints
+//                       overlap: the flush adds with global reductions
+//   bm3d_filter_kernel  the FP32 form (transform 1; explicit fused multiply-adds,
+//                       the library being built without contraction): lane =
+//                       (block, row half); row DCT in registers, column DCT
+//                       through a warp shared buffer, Haar along the group with
+//                       warp shuffles; aggregation into a shared-memory footprint
+//                       of the 8x8 reference tile, then added to the frame
+//                       accumulators.  Tiles are launched in P x P phases so that
+//                       tiles of one launch have disjoint footprints: the flush
+//                       is a plain read-modify-write, no global atomics.
 //   bm3d_basic_kernel   step-1 num/den -> basic estimate + step-2 luminance
 //   bm3d_final_kernel   num/den -> RGB, alpha copied
 #include "bm3d_spec.h"
@@ -1039,8 +1045,8 @@ constexpr int kTcWarps = 8;
 // atomics), so what is not arithmetic counts: block offsets are read four at a
 // time, nothing is staged, the pairs of a segment overlap, and stage 1 keeps two
 // planes (64 registers: four CTAs an SM; stage 2 three).  12 MP chain frame, split
-// products: stage 1 11.3 -> 8.6 ms, stage 2 15.5 -> 12.5 ms against a form with a
-// staging buffer, an offset load and a branch per pair, and a scalar flush.  (The
+// products: stage 1 11.3 -> 8.4 ms, stage 2 15.5 -> 12.5 ms against a form with a
+// staging buffer, an offset load and a branch per pair.  (The
 // products are not merged into MMAs of k = 16: another order of the sums moves
 // coefficients across the threshold.)
 template <int STAGE, bool SPLIT>

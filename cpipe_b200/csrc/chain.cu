@@ -1143,8 +1143,10 @@ static cpipe_cuda_chain* chain_create(const cpipe_cuda_chain_config* cfg, int* s
                 return fail(CPIPE_OOM, c);
             if (cudaMemset(c->d_stats, 0, sizeof(SpotStats)) != cudaSuccess || cudaMemset(c->d_gate, 0, sizeof(int)) != cudaSuccess)
                 return fail(CPIPE_INTERNAL_ERROR, c);
-            // the check runs at the device's highest stream priority, so its small
-            // launches take free SM slots ahead of the network's next layer
+            // the check runs at the device's highest stream priority, so that its
+            // launches start ahead of the network's two kernels, whose CTAs each
+            // fill an SM: the two take turns (12 MP: 1.5 ms and 2.2 ms one after
+            // the other), and the check is done when the network is
             int prio_low = 0, prio_high = 0;
             if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess ||
                 cudaStreamCreateWithPriority(&c->spot_stream, cudaStreamNonBlocking, prio_high) != cudaSuccess ||

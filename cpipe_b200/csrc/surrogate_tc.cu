@@ -40,12 +40,12 @@
 // kernel per layer, 520 so; 1000 frames of 16 x 16: 220, 115 and 84 us.
 //
 // Front kernel: RGBA -> the network's input (the mapping of sg_prep_kernel) by
-// five warps -> layers 0-3 -> bf16 planes.  Back kernel: those planes by bulk
+// four warps -> layers 0-3 -> bf16 planes.  Back kernel: those planes by bulk
 // copies -> layers 4-7 -> residual onto the RGBA frame.
 //
 // Bound by the tensor core's shared-memory reads, (4 + 3) KB per hidden MMA (42
-// KB, 330 clocks, a row of 128 pixels and layer: 74 % of that path's rate in the
-// back kernel, 58 % in the front one), and by the epilogues' latency for the
+// KB, 330 clocks, a row of 128 pixels and layer: 75 % of that path's rate in the
+// back kernel, 58 % in the front one, 2048 x 2048), and by the epilogues' latency for the
 // rest.  Measured, three frames of 1201 x 801: 778 -> 392 us against one kernel
 // per layer with N = 32 (102 us a hidden layer); DRAM traffic 950 -> 152 B/px.
 //
