@@ -84,9 +84,12 @@ __device__ __forceinline__ float rcd_green(const Tap& T) {
     if (dv < dh) return gv;
     return 0.5F * (gh + gv);
 }
+// At any site.  (Selected, not branched to: with the taps loaded under the branch the
+// 12 MP demosaic nodes took 92.9 and 97.1 us, RCD and AMaZE, against 90.9 and 95.3.)
 template <class Tap>
 __device__ __forceinline__ float rcd_green(const Tap& T, int x, int y, const Cfa& cfa) {
-    return cfa.at(x, y) == 1 ? T(0, 0) : rcd_green(T);
+    const float c = T(0, 0), g = rcd_green(T);
+    return cfa.at(x, y) == 1 ? c : g;
 }
 // demosaic_amaze_generator.cpp:24-46, at a red or blue site
 template <class Tap>
@@ -107,7 +110,8 @@ __device__ __forceinline__ float amaze_green(const Tap& T) {
 }
 template <class Tap>
 __device__ __forceinline__ float amaze_green(const Tap& T, int x, int y, const Cfa& cfa) {
-    return cfa.at(x, y) == 1 ? T(0, 0) : amaze_green(T);
+    const float c = T(0, 0), g = amaze_green(T);
+    return cfa.at(x, y) == 1 ? c : g;
 }
 
 // ------------------------------------------------------------ RGBA pixel ops
