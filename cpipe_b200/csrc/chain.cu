@@ -522,9 +522,13 @@ __device__ __forceinline__ void denoise_tone_tile(const Img& in, const Img& out,
             const int by2 = item / (CW / 2), bx2 = item - by2 * (CW / 2);
             const int u = cx0 + 2 * bx2, v = cy0 + 2 * by2;  // unclamped block origin
             const int l = (2 * by2) * CP + 2 * bx2;
-            if (u >= in.w + H || v >= in.h + H) continue;  // further out than any pixel of the frame reads
             Rgba o[4];
-            if (u >= 0 && u + 1 < in.w && v >= 0 && v + 1 < in.h) {
+            if (u >= in.w + H || v >= in.h + H) {
+                // further out than any pixel of the frame reads: any values, but such as the sums
+                // below divide fast (zeros, equal values and what the memory held do not)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) o[k].r = o[k].g = o[k].b = k & 1 ? 0.75F : 0.25F;
+            } else if (u >= 0 && u + 1 < in.w && v >= 0 && v + 1 < in.h) {
                 Rgba q[4];
                 load_pair<T>(in, u, v, &q[0], &q[1]);
                 load_pair<T>(in, u, v + 1, &q[2], &q[3]);
