@@ -1049,7 +1049,8 @@ constexpr int kTcWarps = 8;
 // staging buffer, an offset load and a branch per pair.  (The
 // products are not merged into MMAs of k = 16: another order of the sums moves
 // coefficients across the threshold.)
-template <int STAGE, bool SPLIT>
+// ROWS: the flush adds whole rows (below).
+template <int STAGE, bool SPLIT, bool ROWS>
 __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int ty, int c, int img) {
     extern __shared__ __align__(16) float sm[];
     const int row0 = img * a.h;
@@ -1174,9 +1175,11 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
     // den = map correlated with the Kaiser window (from the kernel arguments), in
     // place: rows, a band at a time, then columns, four columns to a thread (16-byte
     // loads); down the columns a thread keeps the last eight rows in registers.
-    // The frame's sums take whole rows after that: four columns to a thread there,
-    // every lane in another sector, made a small window's stage a tenth slower
-    // (2016 x 1512, 1 x 1 window at step 3: 1210 -> 1077 us; 12 MP default 1 %)
+    // With ROWS the frame's sums take whole rows after that: four columns to a
+    // thread there, every lane in another sector, made a small window's stage a
+    // tenth slower (2016 x 1512, 1 x 1 window at step 3: 1210 -> 1077 us; 12 MP
+    // default 1 %).  The gated kernels add at once: with rows a 12 MP frame that
+    // falls back took 34.77 ms against 34.38.
     const int gx = (fw + 3) / 4, segs = blockDim.x / gx;
     const int seg = threadIdx.x / gx, xx = 4 * (threadIdx.x - seg * gx);
     for (int b0 = 0; b0 < fh; b0 += segs) {
@@ -1195,13 +1198,15 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         if (on) *wr = make_float4(h[0], h[1], h[2], h[3]);
     }
     __syncthreads();
+    float* gn = a.acc + (long long)c * a.npx;
+    float* gd = a.acc + (long long)(3 + c) * a.npx;
     const int seg_rows = (fh + segs - 1) / segs;
     const int y0 = seg * seg_rows, y1 = seg < segs ? min(fh, y0 + seg_rows) : 0;
     float4 r[8];  // r[v]: the row v above
 #pragma unroll
     for (int v = 1; v < 8; ++v)
         r[v] = y0 < y1 && y0 - v >= 0 ? *reinterpret_cast<const float4*>(s_w + (y0 - v) * P + xx) : zero4;
-    __syncthreads();  // the rows above are read: den takes its place in the map
+    if (ROWS) __syncthreads();  // the rows above are read: den takes its place in the map
     for (int yy = y0; yy < y1; ++yy) {
         float4* row = reinterpret_cast<float4*>(s_w + yy * P + xx);
         r[0] = *row;
@@ -1215,11 +1220,22 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
         }
 #pragma unroll
         for (int v = 7; v > 0; --v) r[v] = r[v - 1];
-        *row = d;
+        if constexpr (ROWS) {
+            *row = d;
+        } else {
+            const float4 n = *reinterpret_cast<const float4*>(s_num + yy * P + xx);
+            const long long o = (long long)(fy0 + yy) * a.w + fx0 + xx;
+            const float nv[4] = {n.x, n.y, n.z, n.w}, dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (xx + k < fw && dv[k] > 0.0F) {
+                    atomicAdd(gn + o + k, nv[k]);
+                    atomicAdd(gd + o + k, dv[k]);
+                }
+        }
     }
+    if constexpr (!ROWS) return;
     __syncthreads();
-    float* gn = a.acc + (long long)c * a.npx;
-    float* gd = a.acc + (long long)(3 + c) * a.npx;
     for (int yy = warp; yy < fh; yy += kTcWarps) {
         const long long o = (long long)(fy0 + yy) * a.w + fx0;
         for (int x = lane; x < fw; x += 32) {
@@ -1234,7 +1250,7 @@ __device__ __forceinline__ void filter_tc_tile(const FilterArgs& a, int tx, int 
 
 template <int STAGE, bool SPLIT>
 __global__ void __launch_bounds__(32 * kTcWarps, STAGE == 1 ? 4 : 3) bm3d_filter_tc_kernel(const __grid_constant__ FilterArgs a) {
-    filter_tc_tile<STAGE, SPLIT>(a, blockIdx.x, blockIdx.y, blockIdx.z % 3, blockIdx.z / 3);
+    filter_tc_tile<STAGE, SPLIT, true>(a, blockIdx.x, blockIdx.y, blockIdx.z % 3, blockIdx.z / 3);
 }
 // A gated run seldom happens: a grid of resident CTAs that walk the tiles, so
 // that one which does not costs the launch (3 us) and not the start of every
@@ -1245,7 +1261,7 @@ __global__ void __launch_bounds__(32 * kTcWarps, STAGE == 1 ? 4 : 3) bm3d_filter
     if (gated_off(a.gate)) return;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int z = t / (a.ntx * a.nty), r = t - z * (a.ntx * a.nty);
-        filter_tc_tile<STAGE, SPLIT>(a, r % a.ntx, r / a.ntx, z % 3, z / 3);
+        filter_tc_tile<STAGE, SPLIT, false>(a, r % a.ntx, r / a.ntx, z % 3, z / 3);
         __syncthreads();
     }
 }
