@@ -83,10 +83,12 @@ def test_bm3d_spec_windows_and_ties(cuda_device, h, w, kw, levels):
 
 
 # matching with a thread per reference: either side of its line at steps 1, 3 and 8 (few references), ragged last CTAs,
-# ties throughout, and the line of larger frames (616 x 616 at step 4 has 100 CTAs of 16 x 16: windows below 39)
+# ties throughout, and the line of larger frames (616 x 616 at step 4 has 100 CTAs of 16 x 16: windows below 39).  Flat
+# areas at 0.5 stand on a rounding tie of the 8-bit luminance, which the basic estimate's last bit (the order of float
+# reductions) would decide: one stage there
 @pytest.mark.parametrize("h,w,kw,levels", [
     (41, 50, dict(ns=19, nstep=1), 0), (41, 50, dict(ns=21, nstep=1), 0), (60, 133, dict(ns=25, nstep=3), 0),
-    (60, 133, dict(ns=27, nstep=3), 0), (145, 150, dict(ns=37, nstep=8), 0), (57, 57, dict(ns=3, nstep=3), 2),
+    (60, 133, dict(ns=27, nstep=3), 0), (145, 150, dict(ns=37, nstep=8), 0), (57, 57, dict(ns=3, nstep=3, stages=1), 2),
     (72, 100, dict(ns=21, nstep=3, tau_match1=16000.0, tau_match2=16000.0), 3), (70, 70, dict(ns=9, n2=4), 0),
     (616, 616, dict(ns=37, nstep=4, stages=1), 0)])
 def test_bm3d_spec_small_windows(cuda_device, h, w, kw, levels):
